@@ -14,18 +14,25 @@ constexpr int kMaxMultipoleOrder = 12;
 struct DevLens {
     int type;
     int order;    // multipoles: highest order
+    int same_centre;  // centred where the lens before it (of one launch or sample) is
     double x0, y0;
     float x0h, x0l, y0h, y0l;  // the centre as FP32 pairs: x0 = x0h + x0l to ~2^-48 relative
     float gxh, gxl, gyh, gyl;  // batched sweep: its sample's pixel-grid origin minus the centre
-    // PEMD
-    float q, cth, sth, t, bnorm2, bnorm, qp;  // qp = (1-q^2)/q^2
+    // PEMD: alpha = conj(amp * rs2^h * F(u) * rot / z), see pemd_alpha
+    float cth, sth, q2, cx, cy, amp;
+    int nterms;   // series terms (kSeriesTerms: the full series, complex Horner)
+    int tail;     // some points have |u| >= 0.75
     float an[kSeriesTerms];
-    double an64[kSeriesTerms];
+    double an64[kSeriesTerms], cth64, sth64, cx64, cy64;
+    // power of the squared radius (PEMD and multipoles): h = h0 + h1; general: outside the
+    // range of pow_pos, powf instead
+    float h0, h1;
+    int general;
     // shear
     float ss, c2, s2, gks, cgka, sgka, gss, cgsa, sgsa;
-    // multipoles
-    float alpha, mnorm[kMaxMultipoleOrder + 1], am[kMaxMultipoleOrder + 1],
-        bm[kMaxMultipoleOrder + 1];
+    // multipoles: radial and tangential coefficients of (cos m th, sin m th) per order
+    float rc[kMaxMultipoleOrder + 1], rs[kMaxMultipoleOrder + 1], tc[kMaxMultipoleOrder + 1],
+        ts[kMaxMultipoleOrder + 1];
 };
 
 struct DevLensSet {
@@ -33,81 +40,192 @@ struct DevLensSet {
     DevLens l[kMaxLensesPerLaunch];
 };
 
+// The lens functions take two points at a time, one per half of a float2, so that most of the
+// arithmetic is packed FP32x2 instructions (add, mul, fma on both halves): the deflection is
+// bound by instruction issue, and a pair costs little more than one point.
+__device__ __forceinline__ float2 splat(float a) { return make_float2(a, a); }
+// products with -1 (exact): the packed instructions take no negated operand, and a sign flip
+// of each half costs two
+__device__ __forceinline__ float2 neg2(float2 a) { return __fmul2_rn(a, splat(-1.f)); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b)
+{
+    return __ffma2_rn(b, splat(-1.f), a);
+}
+
 // x - (hi + lo) for FP32 x and a pair (hi, lo), rounded once: Knuth's two-sum gives
 // x - hi = s + e exactly, then s + (e - lo). Exact offsets from a lens centre matter near the
 // centre, where the angle of the offset sets the direction of the deflection; this keeps the
 // FP32 path off the FP64 units, which on GB300 run at a small fraction of the FP32 rate.
-__device__ __forceinline__ float offset_f32(float x, float hi, float lo)
+__device__ __forceinline__ float2 offset_f32(float2 x, float hi, float lo)
 {
-    const float s = x - hi;
-    const float bp = s - x;
-    const float e = (x - (s - bp)) + (-hi - bp);
-    return s + (e - lo);
+    const float2 nh = splat(-hi);
+    const float2 s = __fadd2_rn(x, nh);
+    const float2 bp = sub2(s, x);
+    const float2 e = __fadd2_rn(sub2(x, sub2(s, bp)), sub2(nh, bp));
+    return __fadd2_rn(s, __fadd2_rn(e, splat(-lo)));
 }
 
-__device__ __forceinline__ float2 cmul(float2 a, float2 b)
+// 1 / x by the hardware approximation and one Newton step
+__device__ __forceinline__ float2 recip2(float2 x)
 {
-    return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    float2 r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(x.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(x.y));
+    const float2 e = __ffma2_rn(neg2(x), r, splat(1.f));
+    // the residual is not finite where x is 0, infinite or beyond the approximation's range
+    const float2 n = __ffma2_rn(e, r, r);
+    return make_float2(fabsf(e.x) < 1.f ? n.x : r.x, fabsf(e.y) < 1.f ? n.y : r.y);
 }
 
-__device__ __forceinline__ float2 cdiv(float2 a, float2 b)
+// x^(h0 + h1) for x > 0 and |h0| <= 1: x = 2^e m with m in [1/sqrt 2, sqrt 2),
+// log2 m = f P(f), f = m - 1, the exponent h (e + log2 m) split into an integer n and
+// a rest in [-1/2, 1/2] (h e - n by one fma, so it does not lose the low bits of a large
+// product), 2^rest by a polynomial, 2^n through the exponent field. P (degree 9, 2.1e-9) and
+// the exponential (degree 6, 3.0e-9) are Chebyshev fits of log2(1 + f) / f and 2^y.
+__device__ __forceinline__ float2 pow_pos(float2 x, float h0, float h1)
 {
-    const float d = b.x * b.x + b.y * b.y;
-    const float inv = 1.0f / d;
-    return make_float2((a.x * b.x + a.y * b.y) * inv, (a.y * b.x - a.x * b.y) * inv);
+    const int ix = __float_as_int(x.x), iy = __float_as_int(x.y);
+    const int ex = (ix - 0x3f3504f3) >> 23, ey = (iy - 0x3f3504f3) >> 23;
+    const float2 f = __fadd2_rn(make_float2(__int_as_float(ix - (ex << 23)),
+                                            __int_as_float(iy - (ey << 23))), splat(-1.f));
+    // (float)e through the mantissa of 1.5 * 2^23
+    const float2 e = __fadd2_rn(make_float2(__int_as_float(0x4b400000 + ex),
+                                            __int_as_float(0x4b400000 + ey)),
+                                splat(-12582912.f));
+    float2 p = splat(-0.11021894216537476f);
+    p = __ffma2_rn(p, f, splat(0.18633928894996643f));
+    p = __ffma2_rn(p, f, splat(-0.1910315454006195f));
+    p = __ffma2_rn(p, f, splat(0.20457172393798828f));
+    p = __ffma2_rn(p, f, splat(-0.23961789906024933f));
+    p = __ffma2_rn(p, f, splat(0.28856903314590454f));
+    p = __ffma2_rn(p, f, splat(-0.3606966733932495f));
+    p = __ffma2_rn(p, f, splat(0.4808982014656067f));
+    p = __ffma2_rn(p, f, splat(-0.7213473320007324f));
+    p = __ffma2_rn(p, f, splat(1.4426950216293335f));
+    const float2 l = __fmul2_rn(p, f);  // log2 m
+    const float2 h = splat(h0);
+    const float2 c = __ffma2_rn(h, l, __fmul2_rn(splat(h1), __fadd2_rn(e, l)));
+    const float2 tm = __fadd2_rn(__ffma2_rn(h, e, c), splat(12582912.f));  // rounds to integers
+    const float2 nn = sub2(splat(12582912.f), tm);  // -n
+    const float2 y = __fadd2_rn(__ffma2_rn(h, e, nn), c);
+    float2 r = splat(0.00015472411178052425f);
+    r = __ffma2_rn(r, y, splat(0.0013403140474110842f));
+    r = __ffma2_rn(r, y, splat(0.009618016891181469f));
+    r = __ffma2_rn(r, y, splat(0.055503204464912415f));
+    r = __ffma2_rn(r, y, splat(0.24022650718688965f));
+    r = __ffma2_rn(r, y, splat(0.6931471824645996f));
+    r = __ffma2_rn(r, y, splat(1.f));
+    const float2 sc = make_float2(__int_as_float((__float_as_int(tm.x) << 23) + 0x3f800000),
+                                  __int_as_float((__float_as_int(tm.y) << 23) + 0x3f800000));
+    return __fmul2_rn(r, sc);
 }
 
-// principal square root, branch cut on the negative real axis (C99 csqrt convention)
-__device__ __forceinline__ float2 csqrtf_(float2 z)
+__device__ __forceinline__ float2 lens_power(const DevLens &L, float2 r2)
 {
-    const float r = hypotf(z.x, z.y);
-    float re = sqrtf(0.5f * (r + fabsf(z.x)));
-    float im;
-    if (re == 0.f) return make_float2(0.f, z.y);
-    im = 0.5f * z.y / re;
-    if (z.x >= 0.f) return make_float2(re, im);
-    return make_float2(fabsf(im), copysignf(re, z.y));
-}
-
-__device__ __forceinline__ void pemd_alpha(const DevLens &L, float dx, float dy, float &ax,
-                                           float &ay)
-{
-    // z = ((x-x0) + i(y-y0)) * (cos th' - i sin th')
-    const float2 rot = make_float2(L.cth, -L.sth);
-    const float2 z = cmul(make_float2(dx, dy), rot);
-    const float X = z.x, Y = z.y;
-    const float rs2 = L.q * L.q * X * X + Y * Y;
-    const float rs = sqrtf(rs2);
-    // A = b'^2 / (q z) * (b'/rs)^(t-2)
-    const float pw = powf(L.bnorm / rs, L.t - 2.0f);
-    const float2 A0 = cdiv(make_float2(L.bnorm2, 0.f), make_float2(L.q * z.x, L.q * z.y));
-    const float2 A = make_float2(A0.x * pw, A0.y * pw);
-    // w^2 = q' rs^2 / z^2 ; u = (1 - sqrt(1 - w^2)) / 2
-    const float2 z2 = cmul(z, z);
-    const float2 w2 = cdiv(make_float2(L.qp * rs2, 0.f), z2);
-    const float2 sq = csqrtf_(make_float2(1.0f - w2.x, -w2.y));
-    const float2 u = make_float2(0.5f * (1.0f - sq.x), -0.5f * sq.y);
-    float2 F;
-    if (u.x * u.x + u.y * u.y < 0.5625f) {  // |u| < 0.75: FP32 Horner
-        F = make_float2(L.an[kSeriesTerms - 1], 0.f);
-#pragma unroll
-        for (int n = kSeriesTerms - 2; n >= 0; --n) {
-            F = cmul(F, u);
-            F.x += L.an[n];
-        }
-    } else {  // tail near |u| = 1: series in FP64
-        double fr = L.an64[kSeriesTerms - 1], fi = 0.0;
-        const double ur = u.x, ui = u.y;
-        for (int n = kSeriesTerms - 2; n >= 0; --n) {
-            const double tr = fr * ur - fi * ui;
-            fi = fr * ui + fi * ur;
-            fr = tr + L.an64[n];
-        }
-        F = make_float2((float)fr, (float)fi);
+    if (L.general) {
+        const float h = L.h0 + L.h1;
+        return make_float2(powf(r2.x, h), powf(r2.y, h));
     }
-    const float2 al = cmul(cmul(A, F), rot);
-    ax = al.x;
-    ay = -al.y;  // conj
+    return pow_pos(r2, L.h0, L.h1);
+}
+
+// sum_k an[k] u^k over NT real coefficients at complex u, by synthetic division by
+// (v - u)(v - conj u) = v^2 - 2 Re(u) v + |u|^2: two real multiply-adds per term where complex
+// Horner takes four.
+template <int NT, int NP>
+__device__ __forceinline__ void series_real(const DevLens &L, const float2 (&ur)[NP],
+                                            const float2 (&ui)[NP], float2 (&fr)[NP],
+                                            float2 (&fi)[NP])
+{
+    float2 r[NP], s[NP], b1[NP], b2[NP];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+        r[q] = __fadd2_rn(ur[q], ur[q]);
+        s[q] = neg2(__ffma2_rn(ur[q], ur[q], __fmul2_rn(ui[q], ui[q])));
+        b2[q] = splat(L.an[NT - 1]);
+        b1[q] = __ffma2_rn(r[q], b2[q], splat(L.an[NT - 2]));
+    }
+#pragma unroll
+    for (int k = NT - 3; k >= 1; --k) {
+        const float2 a = splat(L.an[k]);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            const float2 b0 = __ffma2_rn(r[q], b1[q], __ffma2_rn(s[q], b2[q], a));
+            b2[q] = b1[q];
+            b1[q] = b0;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+        fr[q] = __ffma2_rn(b1[q], ur[q], __ffma2_rn(s[q], b2[q], splat(L.an[0])));
+        fi[q] = __fmul2_rn(b1[q], ui[q]);
+    }
+}
+
+// The full series by complex Horner.
+template <int NP>
+__device__ __forceinline__ void series_full(const DevLens &L, const float2 (&ur)[NP],
+                                            const float2 (&ui)[NP], float2 (&fr)[NP],
+                                            float2 (&fi)[NP])
+{
+    float2 nui[NP];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+        nui[q] = neg2(ui[q]);
+        fr[q] = splat(L.an[kSeriesTerms - 1]);
+        fi[q] = splat(0.f);
+    }
+#pragma unroll
+    for (int n = kSeriesTerms - 2; n >= 0; --n) {
+        const float2 a = splat(L.an[n]);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            const float2 tr = __ffma2_rn(fr[q], ur[q], __ffma2_rn(fi[q], nui[q], a));
+            fi[q] = __ffma2_rn(fr[q], ui[q], __fmul2_rn(fi[q], ur[q]));
+            fr[q] = tr;
+        }
+    }
+}
+
+// The series near and beyond |u| = 1 (the tail, q < 0.4), in FP64 from the FP64 offset: there
+// the 20 terms amplify a rounding of u up to 20 times. By synthetic division, as series_real.
+static __device__ __forceinline__ float2 series_tail(const DevLens &L, double dx, double dy)
+{
+    const double X = dx * L.cth64 + dy * L.sth64, Y = dy * L.cth64 - dx * L.sth64;
+    const double inv = 1.0 / (X * X + Y * Y);
+    const double ur = (L.cx64 * X * X + L.cy64 * Y * Y) * inv;
+    const double ui = (L.cy64 - L.cx64) * X * Y * inv;
+    const double r = 2.0 * ur, s = -(ur * ur + ui * ui);
+    double b2 = L.an64[kSeriesTerms - 1], b1 = fma(r, b2, L.an64[kSeriesTerms - 2]);
+    for (int k = kSeriesTerms - 3; k >= 1; --k) {
+        const double b0 = fma(r, b1, fma(s, b2, L.an64[k]));
+        b2 = b1;
+        b1 = b0;
+    }
+    return make_float2((float)fma(b1, ur, fma(s, b2, L.an64[0])), (float)(b1 * ui));
+}
+
+// PEMD. With z = X + iY the offset in the rotated frame and r_s^2 = q^2 X^2 + Y^2, the argument
+// of the series is u = (1 - sqrt(1 - w^2)) / 2, w^2 = (1 - q^2) / q^2 * r_s^2 / z^2. Since
+// z^2 - (1 - q^2) / q^2 r_s^2 = (qX + iY/q)^2 and qX + iY/q has a positive component along z,
+// the principal root is (qX + iY/q) / z exactly, so
+//   u = (cx X + i cy Y) / z,   cx = (1 - q) / 2, cy = (1 - 1/q) / 2,
+// without a complex square root, and |u| <= max(|cx|, |cy|) at every point: the number of
+// series terms that FP32 can tell apart follows from q alone (build_lens). The prefactor
+// b'^2 / (q z) (b' / r_s)^(t - 2) is amp (r_s^2)^h / z, h = (2 - t) / 2, amp = b'^t / q.
+// One reciprocal, of |z|^2, serves both quotients. Gives z, u and a = amp (r_s^2)^h / |z|^2.
+__device__ __forceinline__ void pemd_setup(const DevLens &L, float2 dx, float2 dy, float2 ct,
+                                           float2 st, float2 ns, float2 &X, float2 &Y,
+                                           float2 &ur, float2 &ui, float2 &a)
+{
+    X = __ffma2_rn(dx, ct, __fmul2_rn(dy, st));  // z = (dx + i dy) (cth - i sth)
+    Y = __ffma2_rn(dy, ct, __fmul2_rn(dx, ns));
+    const float2 xx = __fmul2_rn(X, X), yy = __fmul2_rn(Y, Y), xy = __fmul2_rn(X, Y);
+    const float2 pw = lens_power(L, __ffma2_rn(splat(L.q2), xx, yy));
+    const float2 inv = recip2(__fadd2_rn(xx, yy));
+    ur = __fmul2_rn(__ffma2_rn(splat(L.cx), xx, __fmul2_rn(splat(L.cy), yy)), inv);
+    ui = __fmul2_rn(__fmul2_rn(splat(L.cy - L.cx), xy), inv);
+    a = __fmul2_rn(__fmul2_rn(splat(L.amp), pw), inv);
 }
 
 __device__ __forceinline__ void shear_alpha(const DevLens &L, float sx, float sy, float &ax,
@@ -133,54 +251,117 @@ __device__ __forceinline__ void shear_alpha(const DevLens &L, float sx, float sy
     }
 }
 
-__device__ __forceinline__ void multipole_alpha(const DevLens &L, float sx, float sy, float &ax,
-                                                float &ay)
+// Internal multipoles: with e = (sx + i sy) / r, cos m th and sin m th are the parts of e^m
+// (one complex product per order, no angle), and r^(1 - alpha) = (r^2)^h, h = (1 - alpha) / 2.
+template <int NP>
+__device__ __forceinline__ void multipole_alpha(const DevLens &L, const float2 (&sx)[NP],
+                                                const float2 (&sy)[NP], float2 (&ax)[NP],
+                                                float2 (&ay)[NP])
 {
-    const float r = sqrtf(sx * sx + sy * sy);
-    const float th = atan2f(sy, sx);
-    const float cn = sx / r, sn = sy / r;
-    const float rp = powf(r, 1.0f - L.alpha);
-    ax = 0.f;
-    ay = 0.f;
-    for (int m = 3; m <= L.order; ++m) {
-        float sm, cm;
-        sincosf((float)m * th, &sm, &cm);
-        const float dr = -L.mnorm[m] * (2.0f - L.alpha) * rp * (L.bm[m] * sm + L.am[m] * cm);
-        const float dt = L.mnorm[m] * (float)m * rp * (-L.bm[m] * cm + L.am[m] * sm);
-        ax += cn * dr - sn * dt;
-        ay += sn * dr + cn * dt;
+    float2 rp[NP], cn[NP], sn[NP], nsn[NP], cm[NP], sm[NP], dr[NP], dt[NP];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+        const float2 r2 = __ffma2_rn(sx[q], sx[q], __fmul2_rn(sy[q], sy[q]));
+        rp[q] = lens_power(L, r2);
+        float2 ri;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ri.x) : "f"(r2.x));
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ri.y) : "f"(r2.y));
+        // one Newton step: ri += ri (1 - r2 ri^2) / 2
+        const float2 t = __ffma2_rn(neg2(__fmul2_rn(r2, ri)), ri, splat(1.f));
+        ri = __ffma2_rn(__fmul2_rn(splat(0.5f), ri), t, ri);
+        cn[q] = __fmul2_rn(sx[q], ri);
+        sn[q] = __fmul2_rn(sy[q], ri);
+        nsn[q] = neg2(sn[q]);
+        cm[q] = __ffma2_rn(cn[q], cn[q], __fmul2_rn(nsn[q], sn[q]));
+        sm[q] = __fmul2_rn(__fadd2_rn(cn[q], cn[q]), sn[q]);
+        dr[q] = dt[q] = splat(0.f);
     }
-}
-
-template <typename P>
-__device__ __forceinline__ void load_point(const P *pts, long long i, double &x, double &y);
-template <>
-__device__ __forceinline__ void load_point<float2>(const float2 *pts, long long i, double &x,
-                                                   double &y)
-{
-    const float2 v = pts[i];
-    x = v.x;
-    y = v.y;
-}
-template <>
-__device__ __forceinline__ void load_point<double2>(const double2 *pts, long long i, double &x,
-                                                    double &y)
-{
-    const double2 v = pts[i];
-    x = v.x;
-    y = v.y;
+    for (int m = 3; m <= L.order; ++m) {
+        const float2 rc = splat(L.rc[m]), rs = splat(L.rs[m]);
+        const float2 tc = splat(L.tc[m]), ts = splat(L.ts[m]);
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            const float2 c = __ffma2_rn(cm[q], cn[q], __fmul2_rn(sm[q], nsn[q]));
+            sm[q] = __ffma2_rn(cm[q], sn[q], __fmul2_rn(sm[q], cn[q]));
+            cm[q] = c;
+            dr[q] = __ffma2_rn(rc, cm[q], __ffma2_rn(rs, sm[q], dr[q]));
+            dt[q] = __ffma2_rn(tc, cm[q], __ffma2_rn(ts, sm[q], dt[q]));
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NP; ++q) {
+        ax[q] = __fmul2_rn(rp[q], __ffma2_rn(cn[q], dr[q], __fmul2_rn(nsn[q], dt[q])));
+        ay[q] = __fmul2_rn(rp[q], __ffma2_rn(sn[q], dr[q], __fmul2_rn(cn[q], dt[q])));
+    }
 }
 
 // per-lens constants from the reference's packed parameters (host, FP64)
 int build_lens(const lentils_mass_model &m, DevLens &L);
 
-// alpha of one lens at offset (sx, sy) from its centre
-__device__ __forceinline__ void lens_alpha(const DevLens &L, float sx, float sy, float &ax,
-                                           float &ay)
+// alpha of one lens at NP pairs of offsets (sx, sy) from its centre; tail(L, q, h): series_tail
+// of point h of pair q
+template <int NP, class Tail>
+__device__ __forceinline__ void lens_alpha(const DevLens &L, const float2 (&sx)[NP],
+                                           const float2 (&sy)[NP], Tail tail, float2 (&ax)[NP],
+                                           float2 (&ay)[NP])
 {
-    if (L.type == 0) pemd_alpha(L, sx, sy, ax, ay);
-    else if (L.type == 1) shear_alpha(L, sx, sy, ax, ay);
-    else multipole_alpha(L, sx, sy, ax, ay);
+    if (L.type == 0) {
+        float2 fr[NP], fi[NP], ur[NP], ui[NP], X[NP], Y[NP], a[NP];
+        const float2 ct = splat(L.cth), st = splat(L.sth), ns = splat(-L.sth);
+#pragma unroll
+        for (int q = 0; q < NP; ++q)
+            pemd_setup(L, sx[q], sy[q], ct, st, ns, X[q], Y[q], ur[q], ui[q], a[q]);
+        if (L.nterms == 8) {
+            series_real<8, NP>(L, ur, ui, fr, fi);
+        } else if (L.nterms == 12) {
+            series_real<12, NP>(L, ur, ui, fr, fi);
+        } else if (L.nterms == 16) {
+            series_real<16, NP>(L, ur, ui, fr, fi);
+        } else {
+            series_full<NP>(L, ur, ui, fr, fi);
+            if (L.tail) {
+#pragma unroll
+                for (int q = 0; q < NP; ++q) {
+                    if (!(ur[q].x * ur[q].x + ui[q].x * ui[q].x < 0.5625f)) {
+                        const float2 f = tail(L, q, 0);
+                        fr[q].x = f.x;
+                        fi[q].x = f.y;
+                    }
+                    if (!(ur[q].y * ur[q].y + ui[q].y * ui[q].y < 0.5625f)) {
+                        const float2 f = tail(L, q, 1);
+                        fr[q].y = f.x;
+                        fi[q].y = f.y;
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            // alpha = conj(a F conj(z) rot), rot = cth - i sth
+            const float2 gr = __fmul2_rn(a[q], __ffma2_rn(fr[q], X[q], __fmul2_rn(fi[q], Y[q])));
+            const float2 gn = __fmul2_rn(a[q], __ffma2_rn(fr[q], Y[q],
+                                                          neg2(__fmul2_rn(fi[q], X[q]))));
+            ax[q] = __ffma2_rn(gr, ct, __fmul2_rn(gn, ns));
+            ay[q] = __ffma2_rn(gr, st, __fmul2_rn(gn, ct));
+        }
+    } else if (L.type == 1) {
+        if (L.gks == 0.f && L.gss == 0.f) {
+            const float2 sc = splat(L.ss * L.c2), s2 = splat(L.ss * L.s2), nc = neg2(sc);
+#pragma unroll
+            for (int q = 0; q < NP; ++q) {
+                ax[q] = __ffma2_rn(sc, sx[q], __fmul2_rn(s2, sy[q]));
+                ay[q] = __ffma2_rn(s2, sx[q], __fmul2_rn(nc, sy[q]));
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < NP; ++q) {
+                shear_alpha(L, sx[q].x, sy[q].x, ax[q].x, ay[q].x);
+                shear_alpha(L, sx[q].y, sy[q].y, ax[q].y, ay[q].y);
+            }
+        }
+    } else {
+        multipole_alpha<NP>(L, sx, sy, ax, ay);
+    }
 }
 
 }  // namespace lentils

@@ -51,8 +51,15 @@ struct SweepSampleDev {
     float2 *beta_out;
 };
 
-__device__ __forceinline__ void deflect_chunk(const SweepSampleDev &s,
-                                              const DevLens *__restrict__ lenses, int chunk)
+static __device__ __noinline__ float2 pixel_tail(const DevLens &L, const SweepSampleDev &s, int i,
+                                                 int j)
+{
+    return series_tail(L, (s.x0 - L.x0) + i * s.dx, (s.y0 - L.y0) + j * s.dy);
+}
+
+// not inlined: its registers would otherwise push the gridding path into spills
+static __device__ __noinline__ void deflect_chunk(const SweepSampleDev &s,
+                                                  const DevLens *__restrict__ lenses, int chunk)
 {
     const long long npix = (long long)s.nx * s.ny;
     const long long p0 = (long long)chunk * kDeflectChunk;
@@ -64,27 +71,39 @@ __device__ __forceinline__ void deflect_chunk(const SweepSampleDev &s,
     const float dyh = (float)s.dy, dyl = (float)(s.dy - (double)dyh);
     const float xh = (float)s.x0, xl = (float)(s.x0 - (double)xh);
     const float yh = (float)s.y0, yl = (float)(s.y0 - (double)yh);
-    auto pair_sum = [](float ch, float cl, float k, float dh, float dl) {  // (ch+cl) + k(dh+dl)
-        const float pr = k * dh;
-        const float pe = fmaf(k, dh, -pr);
-        const float sm = ch + pr;
-        const float bp = sm - ch;
-        const float e = (ch - (sm - bp)) + (pr - bp);
-        return sm + ((e + pe) + fmaf(k, dl, cl));
+    auto pair_sum = [](float ch, float cl, float2 k, float dh, float dl) {  // (ch+cl) + k(dh+dl)
+        const float2 c = splat(ch), d = splat(dh);
+        const float2 pr = __fmul2_rn(k, d);
+        const float2 pe = __ffma2_rn(k, d, neg2(pr));
+        const float2 sm = __fadd2_rn(c, pr);
+        const float2 bp = sub2(sm, c);
+        const float2 e = __fadd2_rn(sub2(c, sub2(sm, bp)), sub2(pr, bp));
+        return __fadd2_rn(sm, __fadd2_rn(__fadd2_rn(e, pe), __ffma2_rn(k, splat(dl), splat(cl))));
     };
-    for (long long p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
+    // two pixels per thread and step, blockDim.x apart: each store is coalesced
+    for (long long p = p0 + threadIdx.x; p < p1; p += 2 * blockDim.x) {
+        const long long pb = min(p + blockDim.x, npix - 1);
         const int i = (int)(p / s.ny), j = (int)(p - (long long)i * s.ny);
-        float axs = 0.f, ays = 0.f;
+        const int ib = (int)(pb / s.ny), jb = (int)(pb - (long long)ib * s.ny);
+        const float2 ki = make_float2((float)i, (float)ib), kj = make_float2((float)j, (float)jb);
+        float2 axs = splat(0.f), ays = splat(0.f), sx[1], sy[1];
         for (int l = 0; l < s.nlenses; ++l) {
             const DevLens &L = lenses[s.lens0 + l];
-            float ax, ay;
-            lens_alpha(L, pair_sum(L.gxh, L.gxl, (float)i, dxh, dxl),
-                       pair_sum(L.gyh, L.gyl, (float)j, dyh, dyl), ax, ay);
-            axs += ax;
-            ays += ay;
+            float2 ax[1], ay[1];
+            if (!L.same_centre) {
+                sx[0] = pair_sum(L.gxh, L.gxl, ki, dxh, dxl);
+                sy[0] = pair_sum(L.gyh, L.gyl, kj, dyh, dyl);
+            }
+            lens_alpha<1>(L, sx, sy, [&](const DevLens &T, int, int h) {
+                return pixel_tail(T, s, h ? ib : i, h ? jb : j);
+            }, ax, ay);
+            axs = __fadd2_rn(axs, ax[0]);
+            ays = __fadd2_rn(ays, ay[0]);
         }
-        s.beta_out[p] = make_float2(pair_sum(xh, xl, (float)i, dxh, dxl) - axs,
-                                    pair_sum(yh, yl, (float)j, dyh, dyl) - ays);
+        const float2 bx = sub2(pair_sum(xh, xl, ki, dxh, dxl), axs);
+        const float2 by = sub2(pair_sum(yh, yl, kj, dyh, dyl), ays);
+        s.beta_out[p] = make_float2(bx.x, by.x);
+        if (p + blockDim.x < p1) s.beta_out[p + blockDim.x] = make_float2(bx.y, by.y);
     }
 }
 
@@ -269,6 +288,7 @@ int lentils_sweep_create(lentils_sweep **out, const lentils_sweep_sample *in, in
             L.gxl = (float)(gx - (double)L.gxh);
             L.gyh = (float)gy;
             L.gyl = (float)(gy - (double)L.gyh);
+            L.same_centre = l > 0 && L.x0 == hl.back().x0 && L.y0 == hl.back().y0;
             hl.push_back(L);
         }
         if (st) break;

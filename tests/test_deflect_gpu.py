@@ -88,6 +88,44 @@ def test_many_lenses(native):
     check(O.lens_array(models), pts)
 
 
+@pytest.mark.parametrize("q", [0.30, 0.42, 0.556, 0.60, 0.75, 0.9, 0.97, 1.0, 1.3])
+@pytest.mark.parametrize("qh", [0.35, 0.5, 0.7])
+def test_series_lengths_and_pairs(native, q, qh):
+    """Axis ratios on both sides of each length of the series (8, 12, 16 terms and the full
+    series with its FP64 tail), odd point counts and arrays 8 bytes off a 16-byte boundary.
+    Tolerance: about 40 FP32 roundings of 2^-24 per angle, adding at worst linearly (2.4e-6)
+    and in the mean square far below 1e-6; an FP32 position is rounded once more (2^-24 of up
+    to 2.5 arcsec against angles of about 1 arcsec)."""
+    rng = np.random.default_rng(11)
+    lenses = O.lens_array([O.pemd_cpars(1.1, 25.0, q, 0.03, -0.02, qh),
+                           O.shear_cpars(0.03, -0.02, 0.06, 40.0),
+                           O.multipole_cpars(0.03, -0.02, qh, 5, rng.normal(0, 0.02, 6))])
+    for n, off in ((1, 0), (2, 1), (511, 0), (2049, 1)):
+        pts = rng.uniform(-2.5, 2.5, (n + off, 2)).astype(np.float32).astype(np.float64)[off:]
+        ref = pts - O.deflect(lenses, pts)
+        for f32 in (False, True):
+            dt = torch.float32 if f32 else torch.float64
+            whole = torch.zeros((n + off, 2), dtype=dt).cuda()
+            whole[off:] = torch.as_tensor(pts, dtype=dt).cuda()
+            got = gpu_deflect_tensor(lenses, whole[off:])
+            err = (pts - got) - ref
+            assert O.rel_l2(((pts - got)).reshape(-1), ref.reshape(-1)) < 1e-6
+            assert np.max(np.abs(err)) < 2.4e-6 * max(1.0, np.max(np.abs(ref)))
+
+
+def gpu_deflect_tensor(lenses, p):
+    from lentils_gb300 import _native as N
+    L = N.lib()
+    out = torch.empty(p.numel() + 2, dtype=p.dtype, device=p.device)
+    off = 2 if p.data_ptr() % 16 else 0  # the output shares the input's alignment
+    o = out[off:off + p.numel()]
+    fn = L.lentils_deflect_f32 if p.dtype == torch.float32 else L.lentils_deflect_f64io
+    N.check(fn(ctypes.c_void_p(lenses.ctypes.data), len(lenses), ctypes.c_void_p(p.data_ptr()),
+               ctypes.c_void_p(o.data_ptr()), p.numel() // 2,
+               ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    return o.reshape(-1, 2).double().cpu().numpy()
+
+
 def test_singular_centre_gives_nan(native):
     lenses = O.lens_array([O.pemd_cpars(1.0, 30.0, 0.8, 0.05, -0.03, 0.55)])
     pts = np.array([[0.05, -0.03], [0.5, 0.5]])
