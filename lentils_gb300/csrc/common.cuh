@@ -82,6 +82,24 @@ struct KBPoly64 {
     double edge;
 };
 
+// The table of the paired-FP32 form of the FP64 operators (gridding64.cu): degree-11 fits in the
+// even/odd form above, two taps i < w per float2 as in KBPoly, each coefficient as a pair of FP32
+// values, times a factor that makes an axis' weights sum to just under 1 (scale undoes it).
+// eb/ob[0] is the high half of the leading coefficient; eb/ob[k > 0] that of coefficient k plus
+// the tap's bias b (a multiple of b's last place); el/ol the low halves; nb = -b.
+constexpr int kMaxDsTaps = 4;  // largest w
+constexpr int kDsHalf = 6;     // 6 even + 6 odd coefficients
+struct KBPolyDS {
+    float2 eb[kDsHalf][kMaxDsTaps / 2], el[kDsHalf][kMaxDsTaps / 2];
+    float2 ob[kDsHalf][kMaxDsTaps / 2], ol[kDsHalf][kMaxDsTaps / 2];
+    float2 b[kMaxDsTaps / 2], nb[kMaxDsTaps / 2];
+    float peak[2 * kMaxDsTaps];  // bound of each tap's weight
+    double scale2;  // factor of the product of two weights (1 / factor^2)
+    double edge;    // the extra tap's weight, with the factor
+};
+void kb_ds_build(int w, double beta, KBPolyDS *out);
+double kb_profile(double a, double w, double beta);
+
 // Host: fit the table for (w, beta). Returns max abs fit error relative to the peak
 // (evaluated in FP64) through *fit_err when non-null. `out64` may be null.
 void kb_poly_build(int w, double beta, KBPoly *out, double *fit_err, KBPoly64 *out64 = nullptr);
@@ -154,6 +172,7 @@ struct lentils_plan {
     lentils::GridGeom geom;
     lentils::KBPoly kb;
     lentils::KBPoly64 kb64;
+    lentils::KBPolyDS kbds;  // w <= kMaxDsTaps
     int device;
     long long nvis;
     int nrows, nchannels;

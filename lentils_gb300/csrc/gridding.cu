@@ -532,14 +532,22 @@ int launch_grid(const lentils_plan *p, const float2 *vis, float2 *grid, cudaStre
     return launch_grid_r<float>(p, vis, grid, s);
 }
 
+// gridding64.cu
+bool plan_uses_ds(const lentils_plan *p);
+int launch_degrid_ds(const lentils_plan *p, const double2 *grid, double2 *vis, cudaStream_t s,
+                     const double *vscale);
+int launch_grid_ds(const lentils_plan *p, const double2 *vis, double2 *grid, cudaStream_t s);
+
 int launch_degrid64(const lentils_plan *p, const double2 *grid, double2 *vis, cudaStream_t s,
                     const double *vscale)
 {
+    if (p->nitems > 0 && plan_uses_ds(p)) return launch_degrid_ds(p, grid, vis, s, vscale);
     return launch_degrid_r<double>(p, grid, vis, s, vscale);
 }
 
 int launch_grid64(const lentils_plan *p, const double2 *vis, double2 *grid, cudaStream_t s)
 {
+    if (p->nitems > 0 && plan_uses_ds(p)) return launch_grid_ds(p, vis, grid, s);
     return launch_grid_r<double>(p, vis, grid, s);
 }
 

@@ -710,6 +710,7 @@ int lentils_plan_create(lentils_plan **out, const lentils_grid_desc *gd, const d
     p->grid_variant = 0;
     p->degrid_variant = 0;
     kb_poly_build(g.w, gd->kb_beta, &p->kb, nullptr, &p->kb64);
+    if (g.w <= kMaxDsTaps) kb_ds_build(g.w, gd->kb_beta, &p->kbds);
 
     int st = LENTILS_OK;
     if (nvis > 0) st = plan_build(p, uvw, channels, flags, (cudaStream_t)stream);

@@ -55,7 +55,7 @@ double host_bessel_i0(double x)
 
 // Kaiser-Bessel profile on one axis, I0(beta*sqrt(1-(a/w)^2)), zero outside [-w, w]
 // (the per-axis factor of kb_g, lentils/backend/nufft.c:11-21).
-static double kb_profile(double a, double w, double beta)
+double kb_profile(double a, double w, double beta)
 {
     if (!(a >= -w && a <= w)) return 0.0;
     double r = 1.0 - (a / w) * (a / w);
