@@ -16,6 +16,7 @@
 #include <new>
 
 #include "common.cuh"
+#include "fft2d.cuh"
 
 struct lentils_bcb {
     int nx, ny;      // image
@@ -23,6 +24,8 @@ struct lentils_bcb {
     int hy;          // py / 2 + 1
     int padx, pady;  // n / 2
     double centre;   // beam at zero offset
+    bool own = false;  // power-of-two planes: fft2d.cu (real32 / real64 hold its scratch)
+    lentils::Fft2d fft32 = {}, fft64 = {};
     cufftHandle r2c = 0, c2r = 0, d2z = 0, z2d = 0;
     double2 *spec64 = nullptr;  // rfft2(roll(beam)) / (px py)
     float2 *spec32 = nullptr;
@@ -114,6 +117,8 @@ __global__ void crop_kernel(const R *__restrict__ in, R *__restrict__ out, int n
 
 static void bcb_free(lentils_bcb *op)
 {
+    fft2d_free(&op->fft32);
+    fft2d_free(&op->fft64);
     if (op->r2c) cufftDestroy(op->r2c);
     if (op->c2r) cufftDestroy(op->c2r);
     if (op->d2z) cufftDestroy(op->d2z);
@@ -133,18 +138,46 @@ static int bcb_init(lentils_bcb *op, const double *beam, cudaStream_t s)
     LENTILS_CUDA_TRY(cudaMalloc(&op->spec32, sizeof(float2) * nc));
     LENTILS_CUDA_TRY(cudaMalloc(&op->real64, sizeof(double) * nr));
     LENTILS_CUDA_TRY(cudaMalloc(&op->real32, sizeof(float) * nr));
-    LENTILS_CUDA_TRY(cudaMalloc(&op->work64, sizeof(double2) * nc));
-    LENTILS_CUDA_TRY(cudaMalloc(&op->work32, sizeof(float2) * nc));
-    LENTILS_CUFFT_TRY(cufftPlan2d(&op->r2c, op->px, op->py, CUFFT_R2C));
-    LENTILS_CUFFT_TRY(cufftPlan2d(&op->c2r, op->px, op->py, CUFFT_C2R));
-    LENTILS_CUFFT_TRY(cufftPlan2d(&op->d2z, op->px, op->py, CUFFT_D2Z));
-    LENTILS_CUFFT_TRY(cufftPlan2d(&op->z2d, op->px, op->py, CUFFT_Z2D));
+    op->own = fft2d_supported(op->px, op->py);
+    if (op->own) {
+        int st = fft2d_init<float2>(&op->fft32, op->nx, op->ny, op->padx, op->pady, op->px, op->py);
+        if (!st)
+            st = fft2d_init<double2>(&op->fft64, op->nx, op->ny, op->padx, op->pady, op->px, op->py);
+        if (st) return st;
+    } else {
+        LENTILS_CUDA_TRY(cudaMalloc(&op->work64, sizeof(double2) * nc));
+        LENTILS_CUDA_TRY(cudaMalloc(&op->work32, sizeof(float2) * nc));
+        LENTILS_CUFFT_TRY(cufftPlan2d(&op->r2c, op->px, op->py, CUFFT_R2C));
+        LENTILS_CUFFT_TRY(cufftPlan2d(&op->c2r, op->px, op->py, CUFFT_C2R));
+        LENTILS_CUFFT_TRY(cufftPlan2d(&op->d2z, op->px, op->py, CUFFT_D2Z));
+        LENTILS_CUFFT_TRY(cufftPlan2d(&op->z2d, op->px, op->py, CUFFT_Z2D));
+    }
     roll_kernel<<<nblk(nr), 256, 0, s>>>(beam, op->real64, op->px, op->py, op->nx, op->ny);
     LENTILS_CHECK_LAUNCH("roll_kernel");
-    LENTILS_CUFFT_TRY(cufftSetStream(op->d2z, s));
-    LENTILS_CUFFT_TRY(cufftExecD2Z(op->d2z, op->real64, (cufftDoubleComplex *)op->spec64));
+    double2 *mid = nullptr;
+    if (op->own) {  // the beam fills its plane: no padding
+        Fft2d full = op->fft64;
+        full.nx = op->px;
+        full.ny = op->py;
+        full.padx = full.pady = 0;
+        LENTILS_CUDA_TRY(cudaMalloc(&mid, sizeof(double2) * (size_t)op->px * full.pitch));
+        const int st = fft2d_forward<double, double2>(full, op->real64, mid, op->spec64,
+                                                      (const double *)nullptr,
+                                                      (const double *)nullptr, s);
+        if (st) {
+            cudaFree(mid);
+            return st;
+        }
+    } else {
+        LENTILS_CUFFT_TRY(cufftSetStream(op->d2z, s));
+        LENTILS_CUFFT_TRY(cufftExecD2Z(op->d2z, op->real64, (cufftDoubleComplex *)op->spec64));
+    }
     scale_spec_kernel<<<nblk(nc), 256, 0, s>>>(op->spec64, op->spec32, nc, 1.0 / (double)nr);
     LENTILS_CHECK_LAUNCH("scale_spec_kernel");
+    if (mid) {
+        LENTILS_CUDA_TRY(cudaStreamSynchronize(s));
+        LENTILS_CUDA_TRY(cudaFree(mid));
+    }
     LENTILS_CUDA_TRY(cudaMemcpyAsync(&op->centre, beam + (long long)op->nx * op->py + op->ny,
                                      sizeof(double), cudaMemcpyDeviceToHost, s));
     LENTILS_CUDA_TRY(cudaStreamSynchronize(s));
@@ -181,12 +214,18 @@ static int bcb_apply_t(lentils_bcb *op, const R *x, R *out, R *real, C *work, co
 
 int bcb_apply32(lentils_bcb *op, const float *x, float *out, cudaStream_t s)
 {
+    if (op->own)
+        return fft2d_convolve<float, float2>(op->fft32, x, (float2 *)op->real32, op->spec32, out,
+                                             s);
     return bcb_apply_t<float, float2>(op, x, out, op->real32, op->work32, op->spec32, op->r2c,
                                       op->c2r, s);
 }
 
 int bcb_apply64(lentils_bcb *op, const double *x, double *out, cudaStream_t s)
 {
+    if (op->own)
+        return fft2d_convolve<double, double2>(op->fft64, x, (double2 *)op->real64, op->spec64,
+                                               out, s);
     return bcb_apply_t<double, double2>(op, x, out, op->real64, op->work64, op->spec64, op->d2z,
                                         op->z2d, s);
 }

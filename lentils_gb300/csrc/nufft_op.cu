@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fft2d.cuh"
 
 struct lentils_nufft {
     const lentils_plan *plan;
@@ -33,6 +34,9 @@ struct lentils_nufft {
     float2 *grid32;
     double *pad64;
     double2 *grid64;
+    bool own;  // power-of-two planes: the transforms of fft2d.cu, with padding, cropping and
+               // apodisation inside (pad32 / pad64 hold their scratch); else cuFFT
+    lentils::Fft2d fft32, fft64;
     cufftHandle r2c32, c2r32, d2z64, z2d64;
     bool have32, have64;
 };
@@ -144,11 +148,13 @@ static void nufft_free(lentils_nufft *op)
     cudaFree(op->grid32);
     cudaFree(op->pad64);
     cudaFree(op->grid64);
-    if (op->have32) {
+    lentils::fft2d_free(&op->fft32);
+    lentils::fft2d_free(&op->fft64);
+    if (op->have32 && !op->own) {
         cufftDestroy(op->r2c32);
         cufftDestroy(op->c2r32);
     }
-    if (op->have64) {
+    if (op->have64 && !op->own) {
         cufftDestroy(op->d2z64);
         cufftDestroy(op->z2d64);
     }
@@ -182,9 +188,10 @@ int lentils_nufft_create(lentils_nufft **out, const lentils_plan *plan, int nx, 
     op->nv = plan->geom.nv;
     op->half_nv = plan->geom.half_nv;
     op->precisions = precisions;
-    cudaStream_t s = (cudaStream_t)stream;
-    const size_t npad = (size_t)op->nu * op->nv, ngrid = (size_t)op->nu * op->half_nv;
-    int st = LENTILS_OK;
+    (void)stream;
+    const size_t ngrid = (size_t)op->nu * op->half_nv;
+    const size_t npad = std::max((size_t)op->nu * op->nv, 2 * (size_t)nx * fft2d_pitch(op->nv));
+    op->own = fft2d_supported(op->nu, op->nv);
     auto fail = [&](int code) {
         const int c = lentils_last_error();
         char msg[512];
@@ -212,11 +219,13 @@ int lentils_nufft_create(lentils_nufft **out, const lentils_plan *plan, int nx, 
             cuda_status(e, "nufft_create (FP32 buffers)");
             return fail(LENTILS_ERR_CUDA);
         }
-        if (cufftPlan2d(&op->r2c32, op->nu, op->nv, CUFFT_R2C) != CUFFT_SUCCESS) {
+        if (op->own) {
+            if (fft2d_init<float2>(&op->fft32, nx, ny, padx, pady, op->nu, op->nv))
+                return fail(LENTILS_ERR_CUDA);
+        } else if (cufftPlan2d(&op->r2c32, op->nu, op->nv, CUFFT_R2C) != CUFFT_SUCCESS) {
             set_error(LENTILS_ERR_CUDA, "nufft_create: cufftPlan2d R2C");
             return fail(LENTILS_ERR_CUDA);
-        }
-        if (cufftPlan2d(&op->c2r32, op->nu, op->nv, CUFFT_C2R) != CUFFT_SUCCESS) {
+        } else if (cufftPlan2d(&op->c2r32, op->nu, op->nv, CUFFT_C2R) != CUFFT_SUCCESS) {
             cufftDestroy(op->r2c32);
             set_error(LENTILS_ERR_CUDA, "nufft_create: cufftPlan2d C2R");
             return fail(LENTILS_ERR_CUDA);
@@ -236,19 +245,19 @@ int lentils_nufft_create(lentils_nufft **out, const lentils_plan *plan, int nx, 
             cuda_status(e, "nufft_create (FP64 buffers)");
             return fail(LENTILS_ERR_CUDA);
         }
-        if (cufftPlan2d(&op->d2z64, op->nu, op->nv, CUFFT_D2Z) != CUFFT_SUCCESS) {
+        if (op->own) {
+            if (fft2d_init<double2>(&op->fft64, nx, ny, padx, pady, op->nu, op->nv))
+                return fail(LENTILS_ERR_CUDA);
+        } else if (cufftPlan2d(&op->d2z64, op->nu, op->nv, CUFFT_D2Z) != CUFFT_SUCCESS) {
             set_error(LENTILS_ERR_CUDA, "nufft_create: cufftPlan2d D2Z");
             return fail(LENTILS_ERR_CUDA);
-        }
-        if (cufftPlan2d(&op->z2d64, op->nu, op->nv, CUFFT_Z2D) != CUFFT_SUCCESS) {
+        } else if (cufftPlan2d(&op->z2d64, op->nu, op->nv, CUFFT_Z2D) != CUFFT_SUCCESS) {
             cufftDestroy(op->d2z64);
             set_error(LENTILS_ERR_CUDA, "nufft_create: cufftPlan2d Z2D");
             return fail(LENTILS_ERR_CUDA);
         }
         op->have64 = true;
     }
-    (void)s;
-    (void)st;
     *out = op;
     return LENTILS_OK;
 }
@@ -286,6 +295,12 @@ int nufft_forward_scaled(lentils_nufft *op, const float *image, float *vis_plan,
     if (!op || !op->have32 || !image || !vis_plan)
         return set_error(LENTILS_ERR_INVALID, "nufft_forward: bad arguments (FP32 not created?)");
     cudaStream_t s = (cudaStream_t)stream;
+    if (op->own) {
+        if (int st = fft2d_forward<float, float2>(op->fft32, image, (float2 *)op->pad32,
+                                                  op->grid32, op->apx32, op->apy32, s))
+            return st;
+        return launch_degrid(op->plan, op->grid32, (float2 *)vis_plan, s, vscale);
+    }
     LENTILS_CUDA_TRY(pdl_launch(apod_pad_kernel<float>, dim3(nblocks((long long)op->nu * op->nv)), dim3(256), 0, s, image, op->pad32, op->apx32, op->apy32, op->nx, op->ny, op->padx, op->pady, op->nu, op->nv));
     LENTILS_CHECK_LAUNCH("apod_pad_kernel");
     LENTILS_CUFFT_TRY(cufftSetStream(op->r2c32, s));
@@ -300,6 +315,12 @@ int nufft_forward_scaled64(lentils_nufft *op, const double *image, double *vis_p
     if (!op || !op->have64 || !image || !vis_plan)
         return set_error(LENTILS_ERR_INVALID, "nufft_forward64: bad arguments (FP64 not created?)");
     cudaStream_t s = (cudaStream_t)stream;
+    if (op->own) {
+        if (int st = fft2d_forward<double, double2>(op->fft64, image, (double2 *)op->pad64,
+                                                    op->grid64, op->apx64, op->apy64, s))
+            return st;
+        return launch_degrid64(op->plan, op->grid64, (double2 *)vis_plan, s, vscale);
+    }
     LENTILS_CUDA_TRY(pdl_launch(apod_pad_kernel<double>, dim3(nblocks((long long)op->nu * op->nv)), dim3(256), 0, s, image, op->pad64, op->apx64, op->apy64, op->nx, op->ny, op->padx, op->pady, op->nu, op->nv));
     LENTILS_CHECK_LAUNCH("apod_pad_kernel");
     LENTILS_CUFFT_TRY(cufftSetStream(op->d2z64, s));
@@ -319,6 +340,9 @@ int lentils_nufft_adjoint(lentils_nufft *op, const float *vis_plan, float *image
     cudaStream_t s = (cudaStream_t)stream;
     LENTILS_CUDA_TRY(cudaMemsetAsync(op->grid32, 0, sizeof(float2) * (size_t)op->nu * op->half_nv, s));
     if (int st = launch_grid(op->plan, (const float2 *)vis_plan, op->grid32, s)) return st;
+    if (op->own)
+        return fft2d_inverse<float, float2>(op->fft32, op->grid32, (float2 *)op->pad32, image,
+                                            op->apx32, op->apy32, s);
     const int ncols = (op->nv % 2 == 0) ? 2 : 1;
     const int pairs = op->nu / 2 + 1;
     LENTILS_CUDA_TRY(pdl_launch(hermitian_edges_kernel<float2>, dim3((pairs * ncols + 255) / 256), dim3(256), 0, s, op->grid32, op->nu, op->half_nv, ncols, op->half_nv - 1));
@@ -339,6 +363,9 @@ int lentils_nufft_adjoint64(lentils_nufft *op, const double *vis_plan, double *i
     cudaStream_t s = (cudaStream_t)stream;
     LENTILS_CUDA_TRY(cudaMemsetAsync(op->grid64, 0, sizeof(double2) * (size_t)op->nu * op->half_nv, s));
     if (int st = launch_grid64(op->plan, (const double2 *)vis_plan, op->grid64, s)) return st;
+    if (op->own)
+        return fft2d_inverse<double, double2>(op->fft64, op->grid64, (double2 *)op->pad64, image,
+                                              op->apx64, op->apy64, s);
     const int ncols = (op->nv % 2 == 0) ? 2 : 1;
     const int pairs = op->nu / 2 + 1;
     LENTILS_CUDA_TRY(pdl_launch(hermitian_edges_kernel<double2>, dim3((pairs * ncols + 255) / 256), dim3(256), 0, s, op->grid64, op->nu, op->half_nv, ncols, op->half_nv - 1));
