@@ -237,6 +237,7 @@ __global__ void __launch_bounds__(kChunkThreads, 4)
                         const float *__restrict__ vscale)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
+    pdl_entry();
     degrid_item_chunks<W2, K>(grid, coords, out, items[blockIdx.x], item_chunks[blockIdx.x],
                               chunk_begin, kb, g, smraw, vscale);
 }
@@ -250,9 +251,12 @@ static int launch_degrid_t(const lentils_plan *p, const typename Prec<R>::C *gri
         if (p->degrid_variant == 0 && p->chunk_begin && p->chunk_k == 4) {  // the default
             const size_t smem = sizeof(float2) * (size_t)g.E * g.stride;
             if (int st = set_smem(degrid_chunk_kernel<W2, 4>, smem)) return st;
-            degrid_chunk_kernel<W2, 4><<<p->nitems, kChunkThreads, smem, s>>>(
-                grid, p->coords, vis, p->items, p->item_chunks, p->chunk_begin, p->kb, g,
-                vscale);
+            LENTILS_CUDA_TRY(pdl_launch(degrid_chunk_kernel<W2, 4>, dim3(p->nitems),
+                                        dim3(kChunkThreads), smem, s, grid,
+                                        (const uint2 *)p->coords, vis,
+                                        (const WorkItem *)p->items,
+                                        (const int2 *)p->item_chunks,
+                                        (const int *)p->chunk_begin, p->kb, g, vscale));
             LENTILS_CHECK_LAUNCH("degrid_chunk_kernel");
             return LENTILS_OK;
         }
@@ -316,6 +320,7 @@ __global__ void __launch_bounds__(NW * 32)
                       const __grid_constant__ KBPoly kb, const GridGeom g)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
+    pdl_entry();
     grid_rows_item_pairs<W2, NW, NARROW>(vis, coords, grid, items[blockIdx.x], kb, g, smraw);
 }
 
@@ -327,8 +332,9 @@ static int launch_grid_pairs(const lentils_plan *p, const float2 *vis, float2 *g
     const size_t smem = grid_pairs_smem_bytes<W2, NW>(p->geom);
     if (smem > kMaxGridSmem) return LENTILS_OK;
     if (int st = set_smem(grid_pairs_kernel<W2, NW, NARROW>, smem)) return st;
-    grid_pairs_kernel<W2, NW, NARROW><<<p->nitems, NW * 32, smem, s>>>(
-        vis, p->coords, grid, p->items, p->kb, p->geom);
+    LENTILS_CUDA_TRY(pdl_launch(grid_pairs_kernel<W2, NW, NARROW>, dim3(p->nitems), dim3(NW * 32),
+                                smem, s, vis, (const uint2 *)p->coords, grid,
+                                (const WorkItem *)p->items, p->kb, p->geom));
     LENTILS_CHECK_LAUNCH("grid_pairs_kernel");
     *done = true;
     return LENTILS_OK;

@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(kDsThreads, W2 == 6 ? 3 : 4)  // 4 would spill
     unsigned char *rowmax = reinterpret_cast<unsigned char *>(sm + g.E * g.stride);  // E x T
     __shared__ int red[kDsThreads / 32];
     constexpr int w = W2 / 2;
+    pdl_entry();
     const WorkItem it = items[blockIdx.x];
     const int a0 = it.tu * g.T - g.Hu - w, b0 = it.tv * g.T - g.Hv - w;
     const int E = g.E, S = g.stride;
@@ -351,6 +352,7 @@ __global__ void __launch_bounds__(kDsThreads, 3)
     constexpr int G = 32 / W2, NG = NW * G;
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ int red[NW];
+    pdl_entry();
     const WorkItem it = items[blockIdx.x];
     const int E = g.E, S = g.stride;
     float4 *tiles = reinterpret_cast<float4 *>(smraw);
@@ -673,8 +675,9 @@ static int degrid_ds(const lentils_plan *p, const double2 *grid, double2 *vis, c
     const GridGeom &g = p->geom;
     const size_t smem = sizeof(float4) * (size_t)g.E * g.stride + (size_t)g.E * g.T;
     if (int st = ds_smem((const void *)degrid_ds_kernel<W2>, smem)) return st;
-    degrid_ds_kernel<W2><<<p->nitems, kDsThreads, smem, s>>>(grid, p->coords, p->coords_res, vis,
-                                                            p->items, p->kbds, p->geom, vscale);
+    LENTILS_CUDA_TRY(pdl_launch(degrid_ds_kernel<W2>, dim3(p->nitems), dim3(kDsThreads), smem, s,
+                                grid, (const uint2 *)p->coords, (const float2 *)p->coords_res, vis,
+                                (const WorkItem *)p->items, p->kbds, p->geom, vscale));
     LENTILS_CHECK_LAUNCH("degrid_ds_kernel");
     return LENTILS_OK;
 }
@@ -684,8 +687,9 @@ static int grid_ds(const lentils_plan *p, const double2 *vis, double2 *grid, cud
 {
     const size_t smem = grid_ds_smem_bytes<W2>(p->geom);
     if (int st = ds_smem((const void *)grid_ds_kernel<W2>, smem)) return st;
-    grid_ds_kernel<W2><<<p->nitems, kDsThreads, smem, s>>>(vis, p->coords, p->coords_res, grid,
-                                                          p->items, p->kbds, p->geom);
+    LENTILS_CUDA_TRY(pdl_launch(grid_ds_kernel<W2>, dim3(p->nitems), dim3(kDsThreads), smem, s, vis,
+                                (const uint2 *)p->coords, (const float2 *)p->coords_res, grid,
+                                (const WorkItem *)p->items, p->kbds, p->geom));
     LENTILS_CHECK_LAUNCH("grid_ds_kernel");
     return LENTILS_OK;
 }
