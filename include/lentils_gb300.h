@@ -468,8 +468,8 @@ int lentils_tc_timeout_selftest(int *err_dev, int poll_limit, void *stream);
 /* ------------------------------------------------------------------------------------------
  * Batched lens-parameter sweep (no counterpart in the reference, whose operators run one lens
  * model at a time): per sample, deflection of its pixel grid, degridding of its grid and
- * gridding of its visibilities, for all samples in ONE persistent kernel launch (captured in a
- * CUDA graph by lentils_sweep_run with use_graph = 1).
+ * gridding of its visibilities, for all samples in one CUDA graph (lentils_sweep_run with
+ * use_graph = 1) of one kernel per kind of work and Kaiser-Bessel table.
  *
  * Each sample names its plan (KB width 6 or 8; tile and chunk are the plan's), DEVICE buffers
  * in the plan's order and frame as for lentils_degrid / lentils_grid -- grid_in (half plane
@@ -494,18 +494,19 @@ typedef struct {
 } lentils_sweep_sample;
 typedef struct {
     int nsamples;
-    int nwork;        /* work items in the queue                       */
-    int blocks;       /* persistent CTAs (resident slots on all SMs)    */
-    long long smem_bytes;
+    int nwork;        /* work items of all kinds                        */
+    int blocks;       /* CTAs of the persistent forms (resident slots on all SMs) */
+    long long smem_bytes; /* of the persistent forms, per CTA */
     long long total_vis;
     long long total_pixels;
     double algorithmic_bytes; /* per run: 2 x (16 B per visibility + grid) + 8 B per pixel */
 } lentils_sweep_stats;
-/* flags & LENTILS_SWEEP_FORM_MASK: the form of the sweep kernel's items. 0: the ballot gridder
- * and one visibility per degridding thread, three CTAs per SM; 1: the column-pair gridder and
- * same-cell chunk degridding, two CTAs per SM; 2: the column-pair gridder and one visibility
- * per degridding thread, two CTAs per SM. Tuning only: equal results up to FP32 summation
- * order in the grids, identical visibilities. */
+/* flags & LENTILS_SWEEP_FORM_MASK: the form of the sweep. 0: a kernel per kind of work and
+ * table, on three branches of the graph (samples with more than four different tables: one
+ * persistent kernel with the ballot gridder and one visibility per degridding thread, three
+ * CTAs per SM); 1: one persistent kernel with the column-pair gridder and same-cell chunk
+ * degridding, two CTAs per SM; 2: the same with one visibility per degridding thread. Tuning
+ * only: equal results up to FP32 summation order in the grids, identical visibilities. */
 #define LENTILS_SWEEP_FORM_MASK 3
 int lentils_sweep_create(lentils_sweep **sweep, const lentils_sweep_sample *samples, int n,
                          int flags, void *stream);

@@ -1,18 +1,21 @@
 // Batched lens-parameter sweep: hundreds of samples with uneven image sizes and visibility
-// counts go through deflection, degridding and gridding in ONE persistent launch.
+// counts go through deflection, degridding and gridding in one CUDA graph.
 //
 // Every sample brings its own plan (binned visibilities; tile, KB width and chunk chosen per
 // sample), its lens model and its pixel grid. The host flattens all of the samples' work into
-// one queue of items, ordered longest first:
-//   grid    -- one plan work item of a sample: row-owner gridding (grid_rows_item) into the
-//              sample's half-plane grid;
-//   degrid  -- one plan work item of a sample (degrid_item) into plan-order visibilities;
+// lists of items, ordered longest first:
+//   grid    -- one plan work item of a sample into the sample's half-plane grid;
+//   degrid  -- one plan work item of a sample into plan-order visibilities;
 //   deflect -- kDeflectChunk pixels of a sample's grid: beta = theta - sum_l alpha_l(theta).
-// A persistent kernel (one CTA per resident slot on every SM) takes items from the queue with
-// one atomic counter per CTA and item, so big samples spread over the whole GPU and small ones
-// fill the gaps; KB width 6 and 8 items run side by side in the same launch. One run is the
-// counter reset, the zeroing of the samples' output grids and the kernel, captured once in a
-// CUDA graph and replayed.
+//
+// The default form launches one kernel per kind and Kaiser-Bessel table, one CTA per item over
+// all samples, on three branches of the graph (grids: zeroing, then gridding; degridding;
+// deflection), so that big samples spread over the whole GPU and small ones fill the gaps. Each
+// kernel is the single-plan one's item function with the registers it wants and its table in
+// constant memory. One persistent kernel for all kinds (forms 1 and 2, and what samples with more
+// than kMaxGroups tables fall back to) has to hold every path at once: under 80 registers, the
+// limit for three CTAs per SM, the faster item functions spill, and each item stages its table
+// in shared memory. 20 samples, 1.7e7 visibilities: 840 us persistent, 570 us split.
 #include <algorithm>
 #include <new>
 #include <vector>
@@ -107,6 +110,68 @@ static __device__ __noinline__ void deflect_chunk(const SweepSampleDev &s,
     }
 }
 
+// -- the split form -------------------------------------------------------------------------
+constexpr int kMaxGroups = 4;  // Kaiser-Bessel tables with kernels of their own
+
+// A plan work item of a sample, with all that locates it.
+struct SweepItem {
+    int sample, pad;
+    WorkItem it;
+    int2 chunks;  // its same-cell chunks
+};
+
+template <int W2>
+__global__ void __launch_bounds__(128)
+    sweep_grid_kernel(const SweepSampleDev *__restrict__ samples,
+                      const SweepItem *__restrict__ items, const __grid_constant__ KBPoly kb)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const SweepItem d = items[blockIdx.x];
+    const SweepSampleDev &s = samples[d.sample];
+    const GridGeom g = s.g;
+    grid_rows_item_pairs<W2, 4>(s.vis_in, s.coords, s.grid_out, d.it, kb, g, smraw);
+}
+
+template <int W2>
+__global__ void __launch_bounds__(128, 4)
+    sweep_degrid_kernel(const SweepSampleDev *__restrict__ samples,
+                        const SweepItem *__restrict__ items, const __grid_constant__ KBPoly kb)
+{
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const SweepItem d = items[blockIdx.x];
+    const SweepSampleDev &s = samples[d.sample];
+    const GridGeom g = s.g;
+    degrid_item_chunks<W2, 4>(s.grid_in, s.coords, s.vis_out, d.it, d.chunks, s.chunk_begin, kb,
+                              g, smraw);
+}
+
+// work: (sample, chunk) pairs
+__global__ void __launch_bounds__(256)
+    sweep_deflect_kernel(const SweepSampleDev *__restrict__ samples,
+                         const int2 *__restrict__ work, const DevLens *__restrict__ lenses)
+{
+    const int2 w = work[blockIdx.x];
+    deflect_chunk(samples[w.x], lenses, w.y);
+}
+
+// All samples' output grids, kZeroBlocks CTAs each (one launch instead of a memset per sample).
+constexpr int kZeroBlocks = 16;
+__global__ void __launch_bounds__(256) sweep_zero_kernel(const SweepSampleDev *__restrict__ samples)
+{
+    const SweepSampleDev &s = samples[blockIdx.x / kZeroBlocks];
+    if (!s.grid_out) return;
+    const long long n = (long long)s.g.nu * s.g.half_nv;
+    const long long first = (blockIdx.x % kZeroBlocks) * 256LL + threadIdx.x;
+    if (reinterpret_cast<uintptr_t>(s.grid_out) & 15) {
+        for (long long e = first; e < n; e += kZeroBlocks * 256) s.grid_out[e] = make_float2(0.f, 0.f);
+        return;
+    }
+    float4 *p = reinterpret_cast<float4 *>(s.grid_out);
+    for (long long e = first; e < n / 2; e += kZeroBlocks * 256) p[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if ((n & 1) && first == 0) s.grid_out[n - 1] = make_float2(0.f, 0.f);
+}
+
+// -- the persistent forms -------------------------------------------------------------------
 // FORM 0: the ballot gridder and one visibility per degridding thread, three CTAs per SM (80
 // registers, a few bytes of spill). FORM 1: the column-pair gridder and same-cell chunk
 // degridding, two CTAs per SM (128 registers). FORM 2: the column-pair gridder and one
@@ -175,7 +240,20 @@ __global__ void __launch_bounds__(kGridBatch, FORM == 0 ? 3 : 2)
 
 }  // namespace lentils
 
+struct SweepGroup {  // items of one Kaiser-Bessel table
+    lentils::KBPoly kb;
+    int w2, nitems;
+    size_t grid_smem, degrid_smem;
+    lentils::SweepItem *items;
+};
+
 struct lentils_sweep {
+    bool split;  // the split form; else the persistent kernel
+    std::vector<SweepGroup> groups;
+    int2 *chunks;  // deflection work of the split form
+    int nchunks;
+    cudaStream_t side[2];  // its degridding and deflection branches
+    cudaEvent_t fork, join[2];
     int nsamples;
     int nwork;
     int blocks;
@@ -202,6 +280,57 @@ static void sweep_free(lentils_sweep *sw)
     cudaFree(sw->work);
     cudaFree(sw->lenses);
     cudaFree(sw->counter);
+    for (auto &g : sw->groups) cudaFree(g.items);
+    cudaFree(sw->chunks);
+    for (int k = 0; k < 2; ++k) {
+        if (sw->side[k]) cudaStreamDestroy(sw->side[k]);
+        if (sw->join[k]) cudaEventDestroy(sw->join[k]);
+    }
+    if (sw->fork) cudaEventDestroy(sw->fork);
+}
+
+constexpr size_t kMaxSweepSmem = 200 * 1024;
+
+// The limit, not one group's need: groups and sweeps share the kernels.
+template <typename K>
+static cudaError_t sweep_smem_attr(K kern)
+{
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)kMaxSweepSmem);
+}
+
+// The split form's launches, forked from s and joined to it again.
+static int sweep_enqueue_split(lentils_sweep *sw, cudaStream_t s)
+{
+    LENTILS_CUDA_TRY(cudaEventRecord(sw->fork, s));
+    for (int k = 0; k < 2; ++k) LENTILS_CUDA_TRY(cudaStreamWaitEvent(sw->side[k], sw->fork, 0));
+    if (sw->nsamples > 0) {
+        sweep_zero_kernel<<<sw->nsamples * kZeroBlocks, 256, 0, s>>>(sw->samples);
+        LENTILS_CHECK_LAUNCH("sweep_zero_kernel");
+    }
+    for (const SweepGroup &g : sw->groups) {
+        if (g.nitems == 0) continue;
+        if (g.w2 == 8) {
+            sweep_grid_kernel<8><<<g.nitems, 128, g.grid_smem, s>>>(sw->samples, g.items, g.kb);
+            sweep_degrid_kernel<8><<<g.nitems, 128, g.degrid_smem, sw->side[0]>>>(sw->samples,
+                                                                                g.items, g.kb);
+        } else {
+            sweep_grid_kernel<6><<<g.nitems, 128, g.grid_smem, s>>>(sw->samples, g.items, g.kb);
+            sweep_degrid_kernel<6><<<g.nitems, 128, g.degrid_smem, sw->side[0]>>>(sw->samples,
+                                                                                g.items, g.kb);
+        }
+        LENTILS_CHECK_LAUNCH("sweep grid / degrid kernel");
+    }
+    if (sw->nchunks > 0) {
+        sweep_deflect_kernel<<<sw->nchunks, 256, 0, sw->side[1]>>>(sw->samples, sw->chunks,
+                                                                  sw->lenses);
+        LENTILS_CHECK_LAUNCH("sweep_deflect_kernel");
+    }
+    for (int k = 0; k < 2; ++k) {
+        LENTILS_CUDA_TRY(cudaEventRecord(sw->join[k], sw->side[k]));
+        LENTILS_CUDA_TRY(cudaStreamWaitEvent(s, sw->join[k], 0));
+    }
+    return LENTILS_OK;
 }
 
 static cudaError_t sweep_set_smem(int form, int smem)
@@ -223,6 +352,7 @@ static cudaError_t sweep_occupancy(int form, int *per_sm, size_t smem)
 
 static int sweep_enqueue(lentils_sweep *sw, cudaStream_t s)
 {
+    if (sw->split) return sweep_enqueue_split(sw, s);
     LENTILS_CUDA_TRY(cudaMemsetAsync(sw->counter, 0, sizeof(int), s));
     for (auto &z : sw->zero) LENTILS_CUDA_TRY(cudaMemsetAsync(z.first, 0, z.second, s));
     if (sw->nwork > 0) {
@@ -259,6 +389,9 @@ int lentils_sweep_create(lentils_sweep **out, const lentils_sweep_sample *in, in
         delete sw;
         return set_error(LENTILS_ERR_INVALID, "sweep_create: kernel form %d (0 to 2)", flags & 3);
     }
+    sw->split = sw->form == 0;
+    std::vector<std::vector<std::pair<double, SweepItem>>> gitems;  // per group
+    std::vector<std::pair<double, int2>> chunks;
     size_t smem = 0;
     int st = LENTILS_OK;
     for (int k = 0; k < n && !st; ++k) {
@@ -294,10 +427,12 @@ int lentils_sweep_create(lentils_sweep **out, const lentils_sweep_sample *in, in
         if (st) break;
         const long long npix = (long long)a.nx * a.ny;
         sw->total_pixels += npix;
-        for (long long c = 0; c * kDeflectChunk < npix; ++c)
-            items.push_back({(double)std::min<long long>(kDeflectChunk, npix - c * kDeflectChunk) *
-                                 (0.6 + 0.3 * a.nlenses),
-                             SweepWork{k, kSweepDeflect, (int)c, 0}});
+        for (long long c = 0; c * kDeflectChunk < npix; ++c) {
+            const double cost = (double)std::min<long long>(kDeflectChunk, npix - c * kDeflectChunk) *
+                                (0.6 + 0.3 * a.nlenses);
+            items.push_back({cost, SweepWork{k, kSweepDeflect, (int)c, 0}});
+            chunks.push_back({cost, make_int2(k, (int)c)});
+        }
         if (!p) continue;
         const int w2 = 2 * p->geom.w;
         if (w2 != 6 && w2 != 8) {
@@ -344,6 +479,45 @@ int lentils_sweep_create(lentils_sweep **out, const lentils_sweep_sample *in, in
                 break;
             }
         }
+        // the split form: this sample's items join the group of its table
+        std::vector<int2> hchunks(p->nitems);
+        SweepGroup *grp = nullptr;
+        if (p->nitems > 0 && (!p->chunk_begin || p->chunk_k != 4)) sw->split = false;
+        if (sw->split) {
+            size_t q = 0;
+            while (q < sw->groups.size() &&
+                   (sw->groups[q].w2 != w2 || memcmp(&sw->groups[q].kb, &p->kb, sizeof(KBPoly))))
+                ++q;
+            if (q == sw->groups.size()) {
+                if (q == kMaxGroups) {
+                    sw->split = false;
+                } else {
+                    sw->groups.push_back(SweepGroup{p->kb, w2, 0, 0, 0, nullptr});
+                    gitems.emplace_back();
+                }
+            }
+            if (sw->split) {
+                grp = &sw->groups[q];
+                grp->grid_smem = std::max(grp->grid_smem, w2 == 8
+                                                              ? grid_pairs_smem_bytes<8, 4>(p->geom)
+                                                              : grid_pairs_smem_bytes<6, 4>(p->geom));
+                grp->degrid_smem = std::max(grp->degrid_smem, degrid_smem_bytes<float>(p->geom));
+                if (std::max(grp->grid_smem, grp->degrid_smem) > kMaxSweepSmem) sw->split = false;
+                if (p->nitems > 0) {
+                    const cudaError_t e =
+                        cudaMemcpy(hchunks.data(), p->item_chunks, sizeof(int2) * p->nitems,
+                                   cudaMemcpyDeviceToHost);
+                    if (e != cudaSuccess) {
+                        st = cuda_status(e, "sweep_create chunks");
+                        break;
+                    }
+                    for (int i = 0; i < p->nitems; ++i)
+                        gitems[q].push_back({(double)hitems[i].count +
+                                                 0.5 * p->geom.E * p->geom.E,
+                                             SweepItem{k, 0, hitems[i], hchunks[i]}});
+                }
+            }
+        }
         const double tile_cost = (double)p->geom.E * p->geom.E;
         const double taps = (double)w2 * w2;
         for (int i = 0; i < p->nitems; ++i) {
@@ -353,7 +527,7 @@ int lentils_sweep_create(lentils_sweep **out, const lentils_sweep_sample *in, in
         }
     }
     sw->algorithmic_bytes += 8.0 * (double)sw->total_pixels;
-    if (!st && smem > 200 * 1024)
+    if (!st && smem > kMaxSweepSmem)
         st = set_error(LENTILS_ERR_UNSUPPORTED, "sweep_create: %zu bytes of shared memory per item", smem);
     if (st) {
         delete sw;
@@ -379,6 +553,38 @@ int lentils_sweep_create(lentils_sweep **out, const lentils_sweep_sample *in, in
     if (e == cudaSuccess && !hl.empty())
         e = cudaMemcpyAsync(sw->lenses, hl.data(), sizeof(DevLens) * hl.size(), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = sweep_set_smem(sw->form, (int)sw->smem);
+    if (sw->split) {
+        const auto longest = [](const auto &x, const auto &y) { return x.first > y.first; };
+        for (size_t q = 0; q < sw->groups.size() && e == cudaSuccess; ++q) {
+            SweepGroup &g = sw->groups[q];
+            std::stable_sort(gitems[q].begin(), gitems[q].end(), longest);
+            std::vector<SweepItem> h;
+            for (const auto &x : gitems[q]) h.push_back(x.second);
+            g.nitems = (int)h.size();
+            e = cudaMalloc(&g.items, sizeof(SweepItem) * std::max<size_t>(1, h.size()));
+            if (e == cudaSuccess && !h.empty())
+                e = cudaMemcpy(g.items, h.data(), sizeof(SweepItem) * h.size(),
+                               cudaMemcpyHostToDevice);
+            if (e == cudaSuccess)
+                e = g.w2 == 8 ? sweep_smem_attr(sweep_grid_kernel<8>)
+                              : sweep_smem_attr(sweep_grid_kernel<6>);
+            if (e == cudaSuccess)
+                e = g.w2 == 8 ? sweep_smem_attr(sweep_degrid_kernel<8>)
+                              : sweep_smem_attr(sweep_degrid_kernel<6>);
+        }
+        std::stable_sort(chunks.begin(), chunks.end(), longest);
+        std::vector<int2> h;
+        for (const auto &x : chunks) h.push_back(x.second);
+        sw->nchunks = (int)h.size();
+        if (e == cudaSuccess) e = cudaMalloc(&sw->chunks, sizeof(int2) * std::max<size_t>(1, h.size()));
+        if (e == cudaSuccess && !h.empty())
+            e = cudaMemcpy(sw->chunks, h.data(), sizeof(int2) * h.size(), cudaMemcpyHostToDevice);
+        for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
+            e = cudaStreamCreateWithFlags(&sw->side[k], cudaStreamNonBlocking);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sw->join[k], cudaEventDisableTiming);
+        }
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sw->fork, cudaEventDisableTiming);
+    }
     int per_sm = 0, nsm = 0, dev = 0;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);

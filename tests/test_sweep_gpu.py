@@ -92,6 +92,73 @@ def test_sweep_kernel_forms(sweep, form):
         assert torch.equal(other.beta_out[k], sw.beta_out[k]), k
 
 
+@pytest.mark.parametrize("nbeta,sizes", [(1, (33, 20)), (4, (40, 64)), (6, (48, 50))])
+def test_tables_and_odd_grids(nbeta, sizes):
+    """Plans with one, four (the most that get kernels of their own) and six different
+    Kaiser-Bessel tables in one sweep, grids of odd size, a sample without visibilities and one
+    without pixels, output grids 8 bytes off a 16-byte boundary; on the stream and as a graph."""
+    import ctypes
+    from lentils_gb300 import _native as N
+    from lentils_gb300.gridding import GriddingPlan
+    from lentils_gb300.lens_models import ExternalPotential, GlobalLensModel
+    rng = np.random.default_rng(nbeta)
+    lens = GlobalLensModel([ExternalPotential(z=0.5, x=0.0, y=0.0, ss=0.05, sa=20.0)])
+    la = lens.setup_raytracing(2.0)
+    cs, keep = (N.SweepSampleC * (nbeta + 2))(), []
+    for k in range(nbeta + 2):
+        w = 3 if k % 2 else 4
+        four = O.FourierGeom(O.ImageGeom((sizes[k % 2] * 2 + k % 3, sizes[1] * 2 + 1),
+                                         [(-1.0, 1.0), (-1.0, 1.0)]))
+        n = 0 if k == nbeta else 700 + 300 * k
+        uvw = O.synth_uv(rng, n, four, 0.4, w) if n else np.zeros((0, 3))
+        beta = 2.34 * 2 * w * (1 + 0.01 * (k % nbeta))
+        plan = GriddingPlan(uvw, [1.0], four.nu, four.nv, four.du, four.dv, 0.0, 0.0, w, beta,
+                            tile=8 if k % 2 else 16, chunk=256)
+        gi = torch.randn((four.nu, four.half_nv), dtype=torch.complex64, device="cuda")
+        vi = torch.randn(max(1, n), dtype=torch.complex64, device="cuda")
+        go = torch.full((four.nu * four.half_nv + 1,), float("nan"), dtype=torch.complex64,
+                        device="cuda")[k % 2:][:four.nu * four.half_nv]
+        vo = torch.empty_like(vi)
+        nx = 0 if k == nbeta + 1 else 50 + k
+        bo = torch.empty((max(1, nx * nx), 2), dtype=torch.float32, device="cuda")
+        c = cs[k]
+        ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+        c.plan, c.grid_in, c.vis_out, c.vis_in = plan.handle, ptr(gi), ptr(vo), ptr(vi)
+        c.grid_out, c.lenses, c.nlenses = ptr(go), ctypes.c_void_p(la.ctypes.data), len(la)
+        c.nx = c.ny = nx
+        c.x0 = c.y0 = -1.0
+        c.dx = c.dy = 0.04
+        c.beta_out = ptr(bo)
+        keep.append((plan, gi, vi, go, vo, bo, n, nx))
+    h = ctypes.c_void_p()
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    sp = ctypes.c_void_p(st.cuda_stream)
+    N.check(N.lib().lentils_sweep_create(ctypes.byref(h), cs, nbeta + 2, 0, sp))
+    try:
+        for graph in (0, 1, 1):
+            for _, _, _, go, vo, bo, _, _ in keep:
+                go.fill_(float("nan"))
+                vo.zero_()
+                bo.zero_()
+            torch.cuda.synchronize()
+            N.check(N.lib().lentils_sweep_run(h, graph, sp))
+            st.synchronize()
+            for plan, gi, vi, go, vo, bo, n, nx in keep:
+                ref = plan.grid(vi[:n])
+                err = (go.reshape(ref.shape) - ref).abs().norm()
+                assert float(err) <= 1e-6 * float(ref.abs().norm())
+                if n:
+                    assert torch.equal(vo, plan.degrid(gi))
+                if nx:
+                    c = -1.0 + 0.04 * np.arange(nx)
+                    pts = np.stack(np.meshgrid(c, c, indexing="ij"), -1).reshape(-1, 2)
+                    b = lens.deflect(pts, 2.0)
+                    assert np.max(np.abs(bo.cpu().numpy() - b)) < 2e-6
+    finally:
+        N.lib().lentils_sweep_destroy(h)
+
+
 def test_sweep_against_oracle(sweep):
     """Two samples (one per KB width) in user row order against the FP64 CPU oracle."""
     from lentils_gb300.lens_models import GlobalLensModel
