@@ -156,7 +156,13 @@ int build_lens(const lentils_mass_model &m, DevLens &L)
         L.cx64 = 0.5 * (1.0 - qa);
         L.cy64 = 0.5 * (1.0 - 1.0 / qa);
         L.tail = !(std::max(fabs(L.cx64), fabs(L.cy64)) < 0.749);
-        L.amp = (float)(b * b / q * pow(b, t - 2.0));
+        L.q2l = (float)(q * q - (double)L.q2);
+        // the rotation by the rounded (cth, sth) also scales by their norm n: z by n, r_s^2h by
+        // n^2h, 1/z by 1/n and the rotation back by n, n^(2 - t) in all
+        const double n = hypot((double)L.cth, (double)L.sth) / hypot(p[4], p[5]);
+        const double amp = b * b / q * pow(b, t - 2.0) / pow(n, 2.0 - t);
+        L.amp = (float)amp;
+        L.amp1 = L.amp != 0.f ? (float)((amp - (double)L.amp) / (double)L.amp) : 0.f;
         set_power(L, 0.5 * (2.0 - t));
         double an = 1.0;
         for (int n = 0; n < kSeriesTerms; ++n) {
@@ -170,6 +176,8 @@ int build_lens(const lentils_mass_model &m, DevLens &L)
         L.ss = (float)p[2];
         L.c2 = (float)(-p[5] * p[5] + p[4] * p[4]);
         L.s2 = (float)(-2 * p[4] * p[5]);
+        L.ssc = (float)(p[2] * (-p[5] * p[5] + p[4] * p[4]));
+        L.sss = (float)(p[2] * (-2 * p[4] * p[5]));
         L.gks = (float)p[6];
         L.sgka = (float)p[8];
         L.cgka = (float)p[9];

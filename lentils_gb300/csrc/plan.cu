@@ -672,17 +672,30 @@ int lentils_plan_create(lentils_plan **out, const lentils_grid_desc *gd, const d
     memset(p, 0, sizeof(*p));
     p->desc = *gd;
     cudaGetDevice(&p->device);
+    // Tile. A work item pays for its extended tile -- staging or clearing, summing and flushing
+    // (T + 2w)^2 cells -- whatever it holds, so 16-cell tiles win where the grid has many tiles
+    // (2048^2, 1e7 visibilities: degrid + grid 264 us against 300 with 8-cell tiles; 4e5
+    // visibilities: 62 against 99). On a small grid there are too few of them to fill the SMs,
+    // and the ones around the centre are long: 8-cell tiles win up to about 700^2 cells (256^2,
+    // 2e4: 8.4 us against 13.3; 500^2, 1.3e5: 14.9 against 17.1; 512^2, 5e5: 25.7 against 28.6;
+    // 512^2, 2e6: 54.7 against 60.8; 800^2: equal; 1024^2, 5e5: 39.8 against 36.2).
     int T = gd->tile;
-    if (T == 0) T = 16;  // measured best for both kernels (degrid and the row-owner gridder)
+    if (T == 0) T = (long long)gd->nu * gd->nv <= 700LL * 700 ? 8 : 16;
     const int logT = ilog2_exact(T);
     if (logT < 3 || logT > 6) {
         delete p;
         return set_error(LENTILS_ERR_INVALID, "plan_create: tile %d (use 8, 16, 32 or 64)", T);
     }
+    // Work-item size: long items amortise their tile, but the longest must not outlast the rest.
+    // A few hundred items for small problems, four per SM for large ones (256^2, 2e4: 8.4 us with
+    // 64 visibilities, 9.3 with 256; 800^2, 4e5: 30.5 us with 1024, 33.8 with 657, 36.6 with 2048;
+    // 1024^2, 1.6e6 in four channels: 97 us of degrid, grid and frames with 2631, 102 with 1600;
+    // 2048^2, 1e7: 264 us with 4096, 286 with 2048).
     int chunk = gd->chunk;
     if (chunk <= 0) {
-        long long c = nvis / (4LL * 152);
-        chunk = (int)std::max(256LL, std::min(4096LL, c));
+        const long long few = T == 8 ? std::max(64LL, std::min(1024LL, nvis / 300))
+                                     : std::min(1024LL, std::max(256LL, nvis / 64));
+        chunk = (int)std::max(few, std::min(4096LL, T == 8 ? nvis / 1000 : nvis / (4 * 152)));
     }
     p->desc.tile = T;
     p->desc.chunk = chunk;

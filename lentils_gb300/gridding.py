@@ -16,13 +16,21 @@ import torch
 from . import _native as N
 
 
+# Every native argument is declared (argtypes), so plain integers pass as pointers; a c_void_p
+# per argument and a Stream object per call cost more than the call itself.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream_ptr(stream=None):
-    s = torch.cuda.current_stream() if stream is None else stream
-    return ctypes.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return stream.cuda_stream
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 class GriddingPlan:
@@ -165,7 +173,8 @@ class GriddingPlan:
                   stream=None):
         """Plan order c64 -> reference row order (complex128 by default)."""
         if out is None:
-            out = torch.zeros(self.nvis, dtype=dtype, device=vis_plan.device)
+            new = torch.zeros if accumulate else torch.empty  # every value is written
+            out = new(self.nvis, dtype=dtype, device=vis_plan.device)
         c128 = 1 if out.dtype == torch.complex128 else 0
         N.check(N.lib().lentils_vis_from_plan(self._handle, _ptr(vis_plan), _ptr(out), c128,
                                               1 if accumulate else 0, _stream_ptr(stream)))
