@@ -147,6 +147,11 @@ __device__ __forceinline__ void pdl_entry()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// pdl_entry without the early start of the next kernel: for kernels whose CTAs differ in length.
+// A kernel that starts while they drain gets more of its first (longest) CTAs onto the SMs that
+// drain first; dealt out to idle SMs its work is balanced.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <class... KArgs, class... Args>
 inline cudaError_t pdl_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
                               cudaStream_t s, Args &&...args)

@@ -303,11 +303,12 @@ __global__ void __launch_bounds__(kRowPairs<N> *FftShape<N>::T)
     }
 }
 
-// Four columns per CTA. MODE 0: mid (nx rows) -> grid (N rows); 1: grid -> mid (inverse);
-// 2: mid -> mid, forward, times spec, inverse.
+// Four columns per CTA. MODE 0: mid (nx rows) -> grid (N rows); 1: grid -> mid (inverse), and
+// the grid is zero afterwards (the next adjoint accumulates into it without a memset of its
+// own); 2: mid -> mid, forward, times spec, inverse.
 template <typename C, int N, int MODE>
 __global__ void __launch_bounds__(kCols<N> *FftShape<N>::T)
-    fft_columns(const C *in, C *out, const C *__restrict__ spec,
+    fft_columns(C *in, C *out, const C *__restrict__ spec,
                 const C *__restrict__ tw, int nx, int padx, int half, int pitch)
 {
     using S = FftShape<N>;
@@ -326,6 +327,12 @@ __global__ void __launch_bounds__(kCols<N> *FftShape<N>::T)
         v[q].x = v[q].y = 0;
         if (on && (MODE == 1 || (i >= 0 && i < nx)))
             v[q] = in[(long long)i * (MODE == 1 ? half : pitch) + col];
+    }
+    if (MODE == 1 && on) {
+        C zero;
+        zero.x = zero.y = 0;
+#pragma unroll
+        for (int q = 0; q < 16; ++q) in[(long long)(t + q * S::T) * half + col] = zero;
     }
     fft_regs<N, MODE == 1>(v, t, tw, sm);
     if constexpr (MODE == 2) {
@@ -414,7 +421,7 @@ static int rows(const Fft2d &op, bool inverse, const void *in, void *out, const 
 }
 
 template <typename C, int N, int MODE>
-static int columns(const Fft2d &op, const C *in, C *out, const C *spec, cudaStream_t s)
+static int columns(const Fft2d &op, C *in, C *out, const C *spec, cudaStream_t s)
 {
     constexpr int NC = kCols<N>;
     const size_t smem = sizeof(C) * FftShape<N>::PAD * NC;
@@ -444,7 +451,7 @@ static int any_rows(const Fft2d &op, bool inverse, const void *in, void *out, co
 }
 
 template <typename C, int MODE>
-static int any_columns(const Fft2d &op, const C *in, C *out, const C *spec, cudaStream_t s)
+static int any_columns(const Fft2d &op, C *in, C *out, const C *spec, cudaStream_t s)
 {
     switch (op.nu) {
     case 128: return columns<C, 128, MODE>(op, in, out, spec, s);
@@ -465,7 +472,7 @@ int fft2d_forward(const Fft2d &op, const R *img, C *mid, C *grid, const R *apx, 
 }
 
 template <typename R, typename C>
-int fft2d_inverse(const Fft2d &op, const C *grid, C *mid, R *img, const R *apx, const R *apy,
+int fft2d_inverse(const Fft2d &op, C *grid, C *mid, R *img, const R *apx, const R *apy,
                   cudaStream_t s)
 {
     if (int st = any_columns<C, 1>(op, grid, mid, (const C *)nullptr, s)) return st;
@@ -484,7 +491,7 @@ int fft2d_convolve(const Fft2d &op, const R *img, C *mid, const C *spec, R *out,
 #define LENTILS_FFT2D(R, C)                                                                      \
     template int fft2d_forward<R, C>(const Fft2d &, const R *, C *, C *, const R *, const R *,   \
                                      cudaStream_t);                                              \
-    template int fft2d_inverse<R, C>(const Fft2d &, const C *, C *, R *, const R *, const R *,   \
+    template int fft2d_inverse<R, C>(const Fft2d &, C *, C *, R *, const R *, const R *,   \
                                      cudaStream_t);                                              \
     template int fft2d_convolve<R, C>(const Fft2d &, const R *, C *, const C *, R *, cudaStream_t);
 LENTILS_FFT2D(float, float2)

@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(kChunkThreads, 4)
                         const float *__restrict__ vscale)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
-    pdl_entry();
+    pdl_wait();
     degrid_item_chunks<W2, K>(grid, coords, out, items[blockIdx.x], item_chunks[blockIdx.x],
                               chunk_begin, kb, g, smraw, vscale);
 }
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(NW * 32)
                       const __grid_constant__ KBPoly kb, const GridGeom g)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
-    pdl_entry();
+    pdl_wait();
     grid_rows_item_pairs<W2, NW, NARROW>(vis, coords, grid, items[blockIdx.x], kb, g, smraw);
 }
 

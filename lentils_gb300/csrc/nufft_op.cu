@@ -37,6 +37,11 @@ struct lentils_nufft {
     bool own;  // power-of-two planes: the transforms of fft2d.cu, with padding, cropping and
                // apodisation inside (pad32 / pad64 hold their scratch); else cuFFT
     lentils::Fft2d fft32, fft64;
+    // own: the grids that the adjoint accumulates into, zero between calls (fft2d_inverse leaves
+    // them so); not_zero: a call failed in between
+    float2 *acc32;
+    double2 *acc64;
+    bool not_zero32, not_zero64;
     cufftHandle r2c32, c2r32, d2z64, z2d64;
     bool have32, have64;
 };
@@ -148,6 +153,8 @@ static void nufft_free(lentils_nufft *op)
     cudaFree(op->grid32);
     cudaFree(op->pad64);
     cudaFree(op->grid64);
+    cudaFree(op->acc32);
+    cudaFree(op->acc64);
     lentils::fft2d_free(&op->fft32);
     lentils::fft2d_free(&op->fft64);
     if (op->have32 && !op->own) {
@@ -188,7 +195,6 @@ int lentils_nufft_create(lentils_nufft **out, const lentils_plan *plan, int nx, 
     op->nv = plan->geom.nv;
     op->half_nv = plan->geom.half_nv;
     op->precisions = precisions;
-    (void)stream;
     const size_t ngrid = (size_t)op->nu * op->half_nv;
     const size_t npad = std::max((size_t)op->nu * op->nv, 2 * (size_t)nx * fft2d_pitch(op->nv));
     op->own = fft2d_supported(op->nu, op->nv);
@@ -222,6 +228,14 @@ int lentils_nufft_create(lentils_nufft **out, const lentils_plan *plan, int nx, 
         if (op->own) {
             if (fft2d_init<float2>(&op->fft32, nx, ny, padx, pady, op->nu, op->nv))
                 return fail(LENTILS_ERR_CUDA);
+            e = cudaMalloc(&op->acc32, sizeof(float2) * ngrid);
+            if (e == cudaSuccess)
+                e = cudaMemsetAsync(op->acc32, 0, sizeof(float2) * ngrid, (cudaStream_t)stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
+            if (e != cudaSuccess) {
+                cuda_status(e, "nufft_create (FP32 buffers)");
+                return fail(LENTILS_ERR_CUDA);
+            }
         } else if (cufftPlan2d(&op->r2c32, op->nu, op->nv, CUFFT_R2C) != CUFFT_SUCCESS) {
             set_error(LENTILS_ERR_CUDA, "nufft_create: cufftPlan2d R2C");
             return fail(LENTILS_ERR_CUDA);
@@ -248,6 +262,14 @@ int lentils_nufft_create(lentils_nufft **out, const lentils_plan *plan, int nx, 
         if (op->own) {
             if (fft2d_init<double2>(&op->fft64, nx, ny, padx, pady, op->nu, op->nv))
                 return fail(LENTILS_ERR_CUDA);
+            e = cudaMalloc(&op->acc64, sizeof(double2) * ngrid);
+            if (e == cudaSuccess)
+                e = cudaMemsetAsync(op->acc64, 0, sizeof(double2) * ngrid, (cudaStream_t)stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
+            if (e != cudaSuccess) {
+                cuda_status(e, "nufft_create (FP64 buffers)");
+                return fail(LENTILS_ERR_CUDA);
+            }
         } else if (cufftPlan2d(&op->d2z64, op->nu, op->nv, CUFFT_D2Z) != CUFFT_SUCCESS) {
             set_error(LENTILS_ERR_CUDA, "nufft_create: cufftPlan2d D2Z");
             return fail(LENTILS_ERR_CUDA);
@@ -328,6 +350,20 @@ int nufft_forward_scaled64(lentils_nufft *op, const double *image, double *vis_p
     return launch_degrid64(op->plan, op->grid64, (double2 *)vis_plan, s, vscale);
 }
 
+// Adjoint with the transforms of fft2d.cu.
+template <typename R, typename C, class Grid>
+static int own_adjoint(lentils_nufft *op, const Fft2d &fft, C *acc, bool &not_zero, const C *vis,
+                       C *mid, R *image, const R *apx, const R *apy, Grid launch, cudaStream_t s)
+{
+    if (not_zero)  // after a failed call
+        LENTILS_CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(C) * (size_t)op->nu * op->half_nv, s));
+    not_zero = true;
+    if (int st = launch(op->plan, vis, acc, s)) return st;
+    if (int st = fft2d_inverse<R, C>(fft, acc, mid, image, apx, apy, s)) return st;
+    not_zero = false;
+    return LENTILS_OK;
+}
+
 }  // namespace lentils
 
 extern "C" {
@@ -338,11 +374,12 @@ int lentils_nufft_adjoint(lentils_nufft *op, const float *vis_plan, float *image
     if (!op || !op->have32 || !image || !vis_plan)
         return set_error(LENTILS_ERR_INVALID, "nufft_adjoint: bad arguments (FP32 not created?)");
     cudaStream_t s = (cudaStream_t)stream;
+    if (op->own)
+        return own_adjoint<float, float2>(op, op->fft32, op->acc32, op->not_zero32,
+                                          (const float2 *)vis_plan, (float2 *)op->pad32, image,
+                                          op->apx32, op->apy32, launch_grid, s);
     LENTILS_CUDA_TRY(cudaMemsetAsync(op->grid32, 0, sizeof(float2) * (size_t)op->nu * op->half_nv, s));
     if (int st = launch_grid(op->plan, (const float2 *)vis_plan, op->grid32, s)) return st;
-    if (op->own)
-        return fft2d_inverse<float, float2>(op->fft32, op->grid32, (float2 *)op->pad32, image,
-                                            op->apx32, op->apy32, s);
     const int ncols = (op->nv % 2 == 0) ? 2 : 1;
     const int pairs = op->nu / 2 + 1;
     LENTILS_CUDA_TRY(pdl_launch(hermitian_edges_kernel<float2>, dim3((pairs * ncols + 255) / 256), dim3(256), 0, s, op->grid32, op->nu, op->half_nv, ncols, op->half_nv - 1));
@@ -361,11 +398,12 @@ int lentils_nufft_adjoint64(lentils_nufft *op, const double *vis_plan, double *i
     if (!op || !op->have64 || !image || !vis_plan)
         return set_error(LENTILS_ERR_INVALID, "nufft_adjoint64: bad arguments (FP64 not created?)");
     cudaStream_t s = (cudaStream_t)stream;
+    if (op->own)
+        return own_adjoint<double, double2>(op, op->fft64, op->acc64, op->not_zero64,
+                                            (const double2 *)vis_plan, (double2 *)op->pad64,
+                                            image, op->apx64, op->apy64, launch_grid64, s);
     LENTILS_CUDA_TRY(cudaMemsetAsync(op->grid64, 0, sizeof(double2) * (size_t)op->nu * op->half_nv, s));
     if (int st = launch_grid64(op->plan, (const double2 *)vis_plan, op->grid64, s)) return st;
-    if (op->own)
-        return fft2d_inverse<double, double2>(op->fft64, op->grid64, (double2 *)op->pad64, image,
-                                              op->apx64, op->apy64, s);
     const int ncols = (op->nv % 2 == 0) ? 2 : 1;
     const int pairs = op->nu / 2 + 1;
     LENTILS_CUDA_TRY(pdl_launch(hermitian_edges_kernel<double2>, dim3((pairs * ncols + 255) / 256), dim3(256), 0, s, op->grid64, op->nu, op->half_nv, ncols, op->half_nv - 1));
