@@ -700,11 +700,11 @@ __global__ void __launch_bounds__(128, 5)
         }
 #pragma unroll 1
         for (int g = 2 * half0; g < 2 * half1; ++g) {  // 8 channels at a time: 8 g .. 8 g + 7
-            float acc[4][8];
+            float2 acc[4][4];  // pairs of channels
 #pragma unroll
             for (int k = 0; k < 4; ++k)
 #pragma unroll
-                for (int c = 0; c < 8; ++c) acc[k][c] = 0.f;
+                for (int c = 0; c < 4; ++c) acc[k][c] = make_float2(0.f, 0.f);
 #pragma unroll
             for (int t = 0; t < 9; ++t) {
                 const int ky = t / 3, kx = t % 3;
@@ -720,11 +720,10 @@ __global__ void __launch_bounds__(128, 5)
                             for (int px = 0; px < 2; ++px) {
                                 const float xv =
                                     ci ? in1[py + ky][px + kx] : in0[py + ky][px + kx];
-                                float *ac = &acc[py * 2 + px][c4 * 4];
-                                ac[0] = fmaf(xv, wv.x, ac[0]);
-                                ac[1] = fmaf(xv, wv.y, ac[1]);
-                                ac[2] = fmaf(xv, wv.z, ac[2]);
-                                ac[3] = fmaf(xv, wv.w, ac[3]);
+                                const float2 x2 = make_float2(xv, xv);
+                                float2 *ac = &acc[py * 2 + px][c4 * 2];
+                                ac[0] = __ffma2_rn(x2, make_float2(wv.x, wv.y), ac[0]);
+                                ac[1] = __ffma2_rn(x2, make_float2(wv.z, wv.w), ac[1]);
                             }
                     }
                 }
@@ -737,7 +736,8 @@ __global__ void __launch_bounds__(128, 5)
                 bf16 *ub = reinterpret_cast<bf16 *>(&u);
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
-                    const bf16 r = __float2bfloat16(fmaxf(acc[k][c] + bs[g * 8 + c], 0.f));
+                    const float v = (c & 1) ? acc[k][c >> 1].y : acc[k][c >> 1].x;
+                    const bf16 r = __float2bfloat16(fmaxf(v + bs[g * 8 + c], 0.f));
                     ub[c] = r;
                     ps[c] = k == 0 ? bf(r) : ps[c] + bf(r);
                 }
@@ -1275,8 +1275,9 @@ __global__ void __launch_bounds__(kRowThreads)
 
 // Weight and bias gradients of the first layer (2 -> 32 channels, 3 x 3, ReLU) on the CUDA
 // cores: gw[co][t][ci] += sum_p m[p][co] x0[p + off(t)][ci] and gb[co] += sum_p m[p][co], with
-// m = dy masked by y > 0 (dy, y: (Bn, H, W, 32) BF16), x0 the packed 8-channel input (channels
-// 0 and 1), gw in the padded [co][tap][8] layout, taps t = (dh + 1) 3 + dw + 1. A GEMM over
+// m = dy masked by y > 0, dy = bf16(du + 0.25 up2(dp)) (add_pool_grad_kernel's sum, formed here:
+// nothing else reads it; du, y: (Bn, H, W, 32), dp: (Bn, H/2, W/2, 32) BF16), x0 the packed
+// 8-channel input (channels 0 and 1), gw in the padded [co][tap][8] layout, taps t = (dh + 1) 3 + dw + 1. A GEMM over
 // K = pixels would leave the tensor core idle behind transposed copies of dy and x0. A thread
 // owns four output channels (72 products per pixel from one 8-byte gradient load and three new
 // input pairs) and walks runs of kE1Run pixels along a row with the 3 x 3 x 2 input window in
@@ -1284,9 +1285,9 @@ __global__ void __launch_bounds__(kRowThreads)
 // warps in shared memory, and each block adds to gw / gb atomically. W is a multiple of kE1Run.
 constexpr int kE1Run = 16;
 __global__ void __launch_bounds__(256, 2)
-    e1_wgrad_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ y,
-                    const bf16 *__restrict__ x0, float *__restrict__ gw, float *__restrict__ gb,
-                    int Bn, int H, int W)
+    e1_wgrad_kernel(const bf16 *__restrict__ du, const bf16 *__restrict__ dp,
+                    const bf16 *__restrict__ y, const bf16 *__restrict__ x0,
+                    float *__restrict__ gw, float *__restrict__ gb, int Bn, int H, int W)
 {
     tc::pdl_wait();
     tc::pdl_trigger();
@@ -1299,12 +1300,12 @@ __global__ void __launch_bounds__(256, 2)
     for (int q = 0; q < 4; ++q)
 #pragma unroll
         for (int k = 0; k < 18; ++k) acc[q][k] = 0.f;
-    const int wr = W / kE1Run;
-    const long long nruns = (long long)Bn * H * wr;
-    for (long long run = (long long)blockIdx.x * 32 + slot; run < nruns; run += (long long)gridDim.x * 32) {
-        const int w0 = (int)(run % wr) * kE1Run;
-        const long long rh = run / wr;
-        const int h = (int)(rh % H), n = (int)(rh / H);
+    const unsigned wr = W / kE1Run;
+    const unsigned nruns = (unsigned)Bn * H * wr;
+    for (unsigned run = blockIdx.x * 32 + slot; run < nruns; run += gridDim.x * 32) {
+        const unsigned row = run / wr;  // in the stack of images
+        const int w0 = (int)(run - row * wr) * kE1Run;
+        const int n = (int)(row / (unsigned)H), h = (int)row - n * H;
         // loads at clamped addresses, zeroed outside the image, so that they do not depend on
         // branches and the unrolled loop can issue them early
         auto ld = [&](int hh, int ww, float (&v)[2]) {
@@ -1320,20 +1321,24 @@ __global__ void __launch_bounds__(256, 2)
             ld(h - 1 + dh, w0 - 1, xw[dh][0]);
             ld(h - 1 + dh, w0, xw[dh][1]);
         }
-        const size_t o0 = ((size_t)(n * H + h) * W + w0) * 32 + 4 * cq;
+        const size_t o0 = ((size_t)row * W + w0) * 32 + 4 * cq;
+        const size_t p0 = ((size_t)(row >> 1) * (W / 2) + w0 / 2) * 32 + 4 * cq;
 #pragma unroll 2
         for (int k = 0; k < kE1Run; ++k) {
             const int w = w0 + k;
 #pragma unroll
             for (int dh = 0; dh < 3; ++dh) ld(h - 1 + dh, w + 1, xw[dh][2]);
-            const uint2 dd = *reinterpret_cast<const uint2 *>(dy + o0 + k * 32);
+            const uint2 dd = *reinterpret_cast<const uint2 *>(du + o0 + k * 32);
+            const uint2 pp = *reinterpret_cast<const uint2 *>(dp + p0 + (k >> 1) * 32);
             const uint2 yy = *reinterpret_cast<const uint2 *>(y + o0 + k * 32);
             const bf16 *dv = reinterpret_cast<const bf16 *>(&dd);
+            const bf16 *pv = reinterpret_cast<const bf16 *>(&pp);
             const bf16 *yv = reinterpret_cast<const bf16 *>(&yy);
             float m[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                m[q] = bf(yv[q]) > 0.f ? bf(dv[q]) : 0.f;
+                const float d = bf(__float2bfloat16(bf(dv[q]) + 0.25f * bf(pv[q])));
+                m[q] = bf(yv[q]) > 0.f ? d : 0.f;
                 accb[q] += m[q];
             }
 #pragma unroll
@@ -2936,19 +2941,20 @@ static int net_backward(lentils_unet *net, const float *tgt, const float *dout, 
     prep = adj_pool(1, net->d_u2, net->d_p2, net->d_e2, net->e2, H / 2, W / 2, 64);
     if (prep < 0) return set_error(LENTILS_ERR_CUDA, "gradient adjoint launch");
     if ((st = layer_backward(net, 1, net->d_e2, net->e2, net->p1, net->d_p1, Bn, s, prep == 1))) return st;
-    LENTILS_CUDA_TRY(pdl_launch(add_pool_grad_kernel<32>, dim3(blocks_rows(Bn * H)),
-                                dim3(kRowThreads), 0, s, (const bf16 *)net->d_u1,
-                                (const bf16 *)net->d_p1, net->d_e1, Bn * H, W,
-                                (const bf16 *)nullptr, (float *)nullptr));
     if (net->gemm_form == 0 && W % kE1Run == 0) {
         const long long items = np0 / kE1Run / 32;  // block iterations of 32 runs
         const int blocks = (int)std::max(1LL, std::min(items, 152LL * 2));
         LENTILS_CUDA_TRY(pdl_launch(e1_wgrad_kernel, dim3(blocks), dim3(256), 0, s,
-                                    (const bf16 *)net->d_e1, (const bf16 *)net->e1,
-                                    (const bf16 *)net->x0, net->gw_pad[0], net->gb[0], Bn, H, W));
+                                    (const bf16 *)net->d_u1, (const bf16 *)net->d_p1,
+                                    (const bf16 *)net->e1, (const bf16 *)net->x0, net->gw_pad[0],
+                                    net->gb[0], Bn, H, W));
         LENTILS_CHECK_LAUNCH("e1_wgrad_kernel");
-    } else if ((st = layer_backward(net, 0, net->d_e1, net->e1, net->x0, nullptr, Bn, s))) {
-        return st;
+    } else {
+        LENTILS_CUDA_TRY(pdl_launch(add_pool_grad_kernel<32>, dim3(blocks_rows(Bn * H)),
+                                    dim3(kRowThreads), 0, s, (const bf16 *)net->d_u1,
+                                    (const bf16 *)net->d_p1, net->d_e1, Bn * H, W,
+                                    (const bf16 *)nullptr, (float *)nullptr));
+        if ((st = layer_backward(net, 0, net->d_e1, net->e1, net->x0, nullptr, Bn, s))) return st;
     }
     {
         AllLayers P = all_layers(net);
