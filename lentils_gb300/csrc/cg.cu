@@ -36,6 +36,11 @@ int bcb_apply32(lentils_bcb *op, const float *x, float *out, cudaStream_t s);
 int bcb_apply64(lentils_bcb *op, const double *x, double *out, cudaStream_t s);
 double bcb_centre(const lentils_bcb *op);
 int bcb_image_size(const lentils_bcb *op);
+int lensop_apply_t_prior(const lentils_lensop *op, const float *img, const float *s, float *out,
+                         int nx, int ny, double idx2, double idy2, double lambda, cudaStream_t st);
+int lensop_apply_t_prior64(const lentils_lensop *op, const double *img, const double *s,
+                           double *out, int nx, int ny, double idx2, double idy2, double lambda,
+                           cudaStream_t st);
 }  // namespace lentils
 
 struct lentils_normal_op {
@@ -78,10 +83,10 @@ __global__ void scale_vis_kernel(C *__restrict__ v, const R *__restrict__ w, lon
     }
 }
 
-// out (+)= lambda * R^T R s for the forward-difference gradient on an nx x ny grid (x-major).
+// out = lambda * R^T R s for the forward-difference gradient on an nx x ny grid (x-major).
 template <typename R>
 __global__ void rtr_kernel(const R *__restrict__ s, R *__restrict__ out, int nx, int ny, R idx2,
-                           R idy2, R lam, int accumulate)
+                           R idy2, R lam)
 {
     pdl_entry();
     const long long n = (long long)nx * ny;
@@ -94,7 +99,7 @@ __global__ void rtr_kernel(const R *__restrict__ s, R *__restrict__ out, int nx,
         if (i <= nx - 2) acc -= (s[e + ny] - v) * idx2;
         if (j >= 1) acc += (v - s[e - 1]) * idy2;
         if (j <= ny - 2) acc -= (s[e + 1] - v) * idy2;
-        out[e] = (accumulate ? out[e] : (R)0) + lam * acc;
+        out[e] = lam * acc;
     }
 }
 
@@ -733,11 +738,8 @@ int lentils_normal_op_apply(lentils_normal_op *op, const float *s_in, float *out
         if ((st = lentils_nufft_adjoint(op->F, (const float *)op->vis32, op->img32b, stream)))
             return st;
     }
-    if ((st = lentils_lensop_apply_t(op->L, op->img32b, out, stream))) return st;
-    LENTILS_CUDA_TRY(pdl_launch(rtr_kernel<float>, dim3(nb(op->nsrc)), dim3(256), 0, s, s_in, out, op->nsx, op->nsy, (float)op->idx2,
-                                                   (float)op->idy2, (float)op->lambda, 1));
-    LENTILS_CHECK_LAUNCH("rtr_kernel");
-    return LENTILS_OK;
+    return lensop_apply_t_prior(op->L, op->img32b, s_in, out, op->nsx, op->nsy, op->idx2,
+                                 op->idy2, op->lambda, s);
 }
 
 int lentils_normal_op_apply64(lentils_normal_op *op, const double *s_in, double *out,
@@ -757,11 +759,8 @@ int lentils_normal_op_apply64(lentils_normal_op *op, const double *s_in, double 
         if ((st = lentils_nufft_adjoint64(op->F, (const double *)op->vis64, op->img64b, stream)))
             return st;
     }
-    if ((st = lentils_lensop_apply_t64(op->L, op->img64b, out, stream))) return st;
-    LENTILS_CUDA_TRY(pdl_launch(rtr_kernel<double>, dim3(nb(op->nsrc)), dim3(256), 0, s, s_in, out, op->nsx, op->nsy, op->idx2,
-                                                    op->idy2, op->lambda, 1));
-    LENTILS_CHECK_LAUNCH("rtr_kernel");
-    return LENTILS_OK;
+    return lensop_apply_t_prior64(op->L, op->img64b, s_in, out, op->nsx, op->nsy, op->idx2,
+                                   op->idy2, op->lambda, s);
 }
 
 // b = L^T F^T C^-1 d in FP64; d: plan-order plan-frame visibilities (c128, device)
@@ -1166,7 +1165,7 @@ int lentils_prior_gradient_apply(const float *s_in, float *out, int nx, int ny, 
     clear_error();
     if (!s_in || !out || nx < 1 || ny < 1 || !(dx > 0) || !(dy > 0))
         return set_error(LENTILS_ERR_INVALID, "prior_gradient_apply: bad arguments");
-    LENTILS_CUDA_TRY(pdl_launch(rtr_kernel<float>, dim3(nb((long long)nx * ny)), dim3(256), 0, (cudaStream_t)stream, s_in, out, nx, ny, (float)(1.0 / (dx * dx)), (float)(1.0 / (dy * dy)), (float)lambda, 0));
+    LENTILS_CUDA_TRY(pdl_launch(rtr_kernel<float>, dim3(nb((long long)nx * ny)), dim3(256), 0, (cudaStream_t)stream, s_in, out, nx, ny, (float)(1.0 / (dx * dx)), (float)(1.0 / (dy * dy)), (float)lambda));
     LENTILS_CHECK_LAUNCH("rtr_kernel");
     return LENTILS_OK;
 }
@@ -1177,7 +1176,7 @@ int lentils_prior_gradient_apply64(const double *s_in, double *out, int nx, int 
     clear_error();
     if (!s_in || !out || nx < 1 || ny < 1 || !(dx > 0) || !(dy > 0))
         return set_error(LENTILS_ERR_INVALID, "prior_gradient_apply64: bad arguments");
-    LENTILS_CUDA_TRY(pdl_launch(rtr_kernel<double>, dim3(nb((long long)nx * ny)), dim3(256), 0, (cudaStream_t)stream, s_in, out, nx, ny, 1.0 / (dx * dx), 1.0 / (dy * dy), lambda, 0));
+    LENTILS_CUDA_TRY(pdl_launch(rtr_kernel<double>, dim3(nb((long long)nx * ny)), dim3(256), 0, (cudaStream_t)stream, s_in, out, nx, ny, 1.0 / (dx * dx), 1.0 / (dy * dy), lambda));
     LENTILS_CHECK_LAUNCH("rtr_kernel");
     return LENTILS_OK;
 }
