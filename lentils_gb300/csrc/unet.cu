@@ -2168,28 +2168,45 @@ static int conv_persist(const bf16 *act, int C, int ks, int Bn, int H, int W, in
 // 3 x 3 convolution from 32 to 32 channels on a grid 128 pixels wide (c1's forward and data
 // gradient) with input-row reuse. A row tile is one image row; the implicit GEMM of the
 // persistent kernel loads each input row nine times (three taps in each of three output rows,
-// 64-byte box rows), and that L2 -> SM traffic bounds it. Here a CTA takes bands of kRowBand
-// consecutive output rows of one image; each input row of the band (kRowBand + 2 of them) is
-// loaded once, as three boxes shifted by -1, 0, +1 columns (the zero fill at the image edge is
-// the padding), into a ring of kRowSlots slots; the output tile of row h reads its nine A
-// operands from the slots of rows h - 1, h, h + 1, and the slot of row h - 1 is released (MMA
-// commit) after it. The 9 x 32 x 32 weights stay in shared memory. Accumulators double
-// buffered in TMEM and the row epilogues as in tc::gemm_tma_persist_kernel. flip: taps mirrored
-// (data gradient). Warps: 0-3 epilogue, lane 0 of 4 TMA, 5 TMEM + MMA.
-constexpr int kRowBand = 4;
+// 64-byte box rows), and that L2 -> SM traffic bounds it. Here a CTA takes a run of consecutive
+// output rows (of the stack of images, cut where an image ends); each input row of a run (one more
+// at each end) is loaded once, with a column of padding on each side (the zero fill beyond the image
+// edge), into a ring of kRowSlots slots; the output tile of row h reads its nine A operands from
+// the slots of rows h - 1, h, h + 1, the horizontal taps 0, 64 and 128 bytes into the slot (one
+// pixel is one 64-byte row of the swizzled layout, whose chunk permutation goes by the address),
+// and the slot of row h - 1 is released (MMA commit) after it. The 9 x 32 x 32 weights stay in
+// shared memory. Accumulators double buffered in TMEM and the row epilogues as in
+// tc::gemm_tma_persist_kernel. flip: taps mirrored (data gradient). Warps: 0-3 epilogue, lane 0 of
+// 4 TMA, 5 TMEM + MMA. Bound by that traffic, 11 KB per output row and 8 KB out again: 22.7 us
+// forward (with the output layer) and 20.5 us for the data gradient at batch 32 and 128^2; 35.4 and
+// 34.2 with three boxes per input row, one per horizontal tap, in bands of four rows.
+constexpr int kRowsPerSm = 4;  // fewest rows per SM: conv3_rows_ok
 constexpr int kRowSlots = 6;
 struct RowsSmem {
-    static constexpr int kB = 9 * 2048, kVar = 8192, kSlot = 3 * kVar;
+    static constexpr int kB = 9 * 2048, kRow = 130 * 64, kSlot = (kRow + 1023) / 1024 * 1024;
     static constexpr int kBytes = kB + kRowSlots * kSlot + 1024;
 };
+
+// CTA i of g takes rows [T i / g, T (i + 1) / g) of the T rows of a stack of images (or column
+// strips) of H rows: f(image, h0, h1) for each image's part, in order, until it returns false.
+template <class F>
+__device__ __forceinline__ void row_runs(int T, int H, int i, int g, F f)
+{
+    const int q1 = (int)((long long)T * (i + 1) / g);
+    for (int q = (int)((long long)T * i / g); q < q1;) {
+        const int n = q / H, h0 = q - n * H, h1 = min(H, h0 + (q1 - q));
+        if (!f(n, h0, h1)) return;
+        q += h1 - h0;
+    }
+}
 
 template <class EP>
 __global__ void __launch_bounds__(tc::kPersistThreads, 1)
     conv3_rows_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ CUtensorMap mb,
                       const EP ep, int Bn, int H, int flip, int *err)
 {
-    constexpr int S = kRowSlots, R = kRowBand;
-    constexpr int kB = RowsSmem::kB, kVar = RowsSmem::kVar, kSlot = RowsSmem::kSlot;
+    constexpr int S = kRowSlots;
+    constexpr int kB = RowsSmem::kB, kRow = RowsSmem::kRow, kSlot = RowsSmem::kSlot;
     constexpr uint32_t ncols = 64;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ uint64_t bfull, sfull[S], sempty[S], tfull[2], tempty[2], mdone;
@@ -2199,7 +2216,7 @@ __global__ void __launch_bounds__(tc::kPersistThreads, 1)
     unsigned char *smem = smem_raw + ((1024 - (tc::smem_u32(smem_raw) & 1023)) & 1023);
     unsigned char *bres = smem, *slots = smem + kB;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int bpi = (H + R - 1) / R, nbands = Bn * bpi;
+    const int rows = Bn * H;
 
     if (warp == 5) {
         tc::tmem_alloc(&tmem_base, ncols);
@@ -2236,22 +2253,18 @@ __global__ void __launch_bounds__(tc::kPersistThreads, 1)
             tc::mbar_arrive_expect_tx(&bfull, 9 * 2048);
             for (int t = 0; t < 9; ++t) tc::tma_load_2d(bres + t * 2048, &mb, t * 32, 0, &bfull);
             int L = 0;
-            bool ok = true;
-            for (int b = blockIdx.x; b < nbands && ok; b += gridDim.x) {
-                const int n = b / bpi, h0 = (b - n * bpi) * R, h1 = min(H, h0 + R);
+            row_runs(rows, H, blockIdx.x, gridDim.x, [&](int n, int h0, int h1) {
                 for (int r = h0 - 1; r <= h1; ++r, ++L) {
                     const int sl = L % S;
                     if (L >= S && !tc::mbar_wait(&sempty[sl], ((L / S) - 1) & 1)) {
                         atomicExch(&abort_flag, 1);
-                        ok = false;
-                        break;
+                        return false;
                     }
-                    unsigned char *dst = slots + sl * kSlot;
-                    tc::mbar_arrive_expect_tx(&sfull[sl], 3 * kVar);
-#pragma unroll
-                    for (int v = 0; v < 3; ++v) tc::tma_load_4d(dst + v * kVar, &ma, 0, v - 1, r, n, &sfull[sl]);
+                    tc::mbar_arrive_expect_tx(&sfull[sl], kRow);
+                    tc::tma_load_4d(slots + sl * kSlot, &ma, 0, -1, r, n, &sfull[sl]);
                 }
-            }
+                return true;
+            });
             if (!tc::mbar_wait(&bfull, 0)) atomicExch(&abort_flag, 1);
 #pragma unroll 1
             for (int i = 0; i < S; ++i) {
@@ -2267,23 +2280,16 @@ __global__ void __launch_bounds__(tc::kPersistThreads, 1)
             bool ok = tc::mbar_wait(&bfull, 0);
             tc::tc_fence_after();
             int L = 0, j = 0;
-            for (int b = blockIdx.x; b < nbands && ok; b += gridDim.x) {
-                const int n = b / bpi, h0 = (b - n * bpi) * R, h1 = min(H, h0 + R);
-                (void)n;
+            if (ok) row_runs(rows, H, blockIdx.x, gridDim.x, [&](int, int h0, int h1) {
                 const int nrows = h1 - h0 + 2;
-                int ready = 0;  // loads of this band known to have landed
-                for (int h = h0; h < h1 && ok; ++h, ++j) {
+                int ready = 0;  // loads of this run known to have landed
+                for (int h = h0; h < h1; ++h, ++j) {
                     const int buf = j & 1;
-                    if (j >= 2 && !tc::mbar_wait(&tempty[buf], ((j >> 1) - 1) & 1)) {
-                        ok = false;
-                        break;
-                    }
-                    while (ok && ready <= h - h0 + 2) {
+                    if (j >= 2 && !tc::mbar_wait(&tempty[buf], ((j >> 1) - 1) & 1)) return ok = false;
+                    for (; ready <= h - h0 + 2; ++ready) {
                         const int Lr = L + ready;
-                        ok = tc::mbar_wait(&sfull[Lr % S], (Lr / S) & 1);
-                        ++ready;
+                        if (!tc::mbar_wait(&sfull[Lr % S], (Lr / S) & 1)) return ok = false;
                     }
-                    if (!ok) break;
                     tc::tc_fence_after();
                     const uint32_t acc = tmem + (uint32_t)(buf * 32);
 #pragma unroll
@@ -2294,7 +2300,7 @@ __global__ void __launch_bounds__(tc::kPersistThreads, 1)
                             dw = -dw;
                         }
                         const int Lr = L + (h + dh) - (h0 - 1);
-                        const uint32_t a = tc::smem_u32(slots + (Lr % S) * kSlot + (dw + 1) * kVar);
+                        const uint32_t a = tc::smem_u32(slots + (Lr % S) * kSlot + (dw + 1) * 64);
                         const uint32_t bb = tc::smem_u32(bres + t * 2048);
 #pragma unroll
                         for (int k = 0; k < 2; ++k)
@@ -2304,11 +2310,11 @@ __global__ void __launch_bounds__(tc::kPersistThreads, 1)
                     tc::mma_commit(&tfull[buf]);
                     tc::mma_commit(&sempty[(L + h - h0) % S]);  // row h - 1: no later tile reads it
                 }
-                if (!ok) break;
                 tc::mma_commit(&sempty[(L + nrows - 2) % S]);
                 tc::mma_commit(&sempty[(L + nrows - 1) % S]);
                 L += nrows;
-            }
+                return true;
+            });
             if (!ok) atomicExch(&abort_flag, 1);
             tc::mma_commit(&mdone);
             if (!tc::mbar_wait(&mdone, 0)) atomicExch(&abort_flag, 1);
@@ -2317,9 +2323,7 @@ __global__ void __launch_bounds__(tc::kPersistThreads, 1)
     } else {  // the epilogue warps
         const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
         int j = 0;
-        bool go_on = true;
-        for (int b = blockIdx.x; b < nbands && go_on; b += gridDim.x) {
-            const int n = b / bpi, h0 = (b - n * bpi) * R, h1 = min(H, h0 + R);
+        row_runs(rows, H, blockIdx.x, gridDim.x, [&](int n, int h0, int h1) {
             for (int h = h0; h < h1; ++h, ++j) {
                 const int buf = j & 1;
                 int go = 0;
@@ -2328,8 +2332,7 @@ __global__ void __launch_bounds__(tc::kPersistThreads, 1)
                 go = __shfl_sync(0xffffffffu, go, 0);
                 if (!go) {
                     if (lane == 0) atomicExch(&abort_flag, 1);
-                    go_on = false;
-                    break;
+                    return false;
                 }
                 tc::tc_fence_after();
                 const int m = ((n * H + h) << 7) + warp * 32 + lane;
@@ -2345,7 +2348,8 @@ __global__ void __launch_bounds__(tc::kPersistThreads, 1)
                 ep.row(m, 0, v, acc, scratch);
                 ep.row_end(m, acc, scratch);
             }
-        }
+            return true;
+        });
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -2370,7 +2374,7 @@ static int conv3_rows_launch(const bf16 *act, int Bn, int H, int flip, const bf1
     CUtensorMap ma, mb;
     const uint64_t da[4] = {(uint64_t)C, (uint64_t)W, (uint64_t)H, (uint64_t)Bn};
     const uint64_t sa[3] = {(uint64_t)C * 2, (uint64_t)W * C * 2, (uint64_t)H * W * C * 2};
-    const uint32_t ba[4] = {32, 128, 1, 1};
+    const uint32_t ba[4] = {32, W + 2, 1, 1};
     if (int st = tma_map_bf16(&ma, act, 4, da, sa, ba, 64)) return st;
     const uint64_t db[2] = {288, 32};
     const uint64_t sb[1] = {288 * 2};
@@ -2378,21 +2382,20 @@ static int conv3_rows_launch(const bf16 *act, int Bn, int H, int flip, const bf1
     if (int st = tma_map_bf16(&mb, wt, 2, db, sb, bb, 64)) return st;
     const PersistShape &shape = conv3_rows_shape<EP>();
     LENTILS_CUDA_TRY(shape.err);
-    const int nbands = Bn * ((H + kRowBand - 1) / kRowBand);
-    const int grid = std::min(nbands, std::max(1, num_sms() * shape.per_sm));
+    const int grid = std::min(Bn * H, std::max(1, num_sms() * shape.per_sm));
     LENTILS_CUDA_TRY(pdl_launch(conv3_rows_kernel<EP>, dim3(grid), dim3(tc::kPersistThreads),
                                 (size_t)RowsSmem::kBytes, s, ma, mb, ep, Bn, H, flip, err));
     LENTILS_CHECK_LAUNCH("conv3_rows_kernel");
     return LENTILS_OK;
 }
 
-// the band kernel for a convolution of Bn images of H x W: the shape it takes, and enough bands
-// (kRowBand rows each) to give every SM one; with fewer (batch 1) the persistent GEMM's
-// row tiles spread wider
+// the row kernel for a convolution of Bn images of H x W: the shape it takes, and at least
+// kRowsPerSm rows of each image for every SM (a run of fewer rows loads more halo than it reuses);
+// with fewer (batch 1) the persistent GEMM's row tiles spread wider
 static bool conv3_rows_ok(int C, int N, int ks, int W, int Bn, int H)
 {
     return C == 32 && N == 32 && ks == 3 && W == 128 &&
-           (long long)Bn * ((H + kRowBand - 1) / kRowBand) >= num_sms();
+           (long long)Bn * ((H + kRowsPerSm - 1) / kRowsPerSm) >= num_sms();
 }
 
 // whether a layer's convolution can take the TMA operands: row tiles of 128 pixels inside one
