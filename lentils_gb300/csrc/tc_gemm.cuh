@@ -430,6 +430,7 @@ __global__ void __launch_bounds__(kPipeThreads)
         }
     } else if (threadIdx.x == 128) {  // the MMA issuer
         constexpr uint32_t idesc = idesc_bf16_f32(128, N);
+        const uint64_t d0 = smem_desc_swz<SWZ>(smem_u32(smem));
         for (int ch = 0; ch < nchunks; ++ch) {
             const int st = ch % STAGES;
             if (!mbar_wait(&full[st], (ch / STAGES) & 1) || *(volatile int *)&abort_flag) {
@@ -437,12 +438,11 @@ __global__ void __launch_bounds__(kPipeThreads)
                 break;
             }
             tc_fence_after();
-            const uint32_t sa = smem_u32(smem + st * kStage);
-            const uint32_t sb = sa + kATile;
+            const uint64_t da = desc_step(d0, st * kStage), db = desc_step(da, kATile);
 #pragma unroll
             for (int k = 0; k < KCH / 16; ++k)
-                mma_bf16(tmem, smem_desc_swz<SWZ>(sa + 32 * k), smem_desc_swz<SWZ>(sb + 32 * k),
-                         idesc, (ch > 0 || k > 0) ? 1u : 0u);
+                mma_bf16(tmem, desc_step(da, 32 * k), desc_step(db, 32 * k), idesc,
+                         (ch > 0 || k > 0) ? 1u : 0u);
             mma_commit(&empty[st]);
         }
         mma_commit(&done);
@@ -608,7 +608,8 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
     } else if (warp == 5) {
         if (lane == 0) {  // the MMA issuer
             constexpr uint32_t idesc = idesc_bf16_f32(128, N);
-            int it = 0;
+            const uint64_t d0 = smem_desc_swz<SWZ>(smem_u32(smem));
+            int st = 0, phase = 0;
             bool ok = true;
             for (int j = 0; j < ntiles && ok; ++j) {
                 const int buf = j & 1;
@@ -618,21 +619,23 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
                 }
                 tc_fence_after();
                 const uint32_t acc = tmem + (uint32_t)(buf * N);
-                for (int ch = 0; ch < nchunks; ++ch, ++it) {
-                    const int st = it % STAGES;
-                    if (!mbar_wait(&full[st], (it / STAGES) & 1)) {
+                for (int ch = 0; ch < nchunks; ++ch) {
+                    if (!mbar_wait(&full[st], phase)) {
                         atomicExch(&abort_flag, 1);
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sa = smem_u32(smem + st * kStage);
-                    const uint32_t sb = sa + kATile;
+                    const uint64_t da = desc_step(d0, st * kStage), db = desc_step(da, kATile);
 #pragma unroll
                     for (int k = 0; k < KCH / 16; ++k)
-                        mma_bf16(acc, smem_desc_swz<SWZ>(sa + 32 * k), smem_desc_swz<SWZ>(sb + 32 * k),
-                                 idesc, (ch > 0 || k > 0) ? 1u : 0u);
+                        mma_bf16(acc, desc_step(da, 32 * k), desc_step(db, 32 * k), idesc,
+                                 (ch > 0 || k > 0) ? 1u : 0u);
                     mma_commit(&empty[st]);
+                    if (++st == STAGES) {
+                        st = 0;
+                        phase ^= 1;
+                    }
                 }
                 if (ok) mma_commit(&tfull[buf]);
             }

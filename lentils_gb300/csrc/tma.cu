@@ -29,18 +29,15 @@ static int encoder(PfnEncodeTiled *out)
     return LENTILS_OK;
 }
 
-int tma_map_bf16(CUtensorMap *map, const void *base, int rank, const uint64_t *dims,
-                 const uint64_t *strides, const uint32_t *box, int swizzle)
+static int encode(CUtensorMap *map, CUtensorMapDataType type, CUtensorMapSwizzle swizzle,
+                  const void *base, int rank, const uint64_t *dims, const uint64_t *strides,
+                  const uint32_t *box)
 {
-    if (swizzle != 64 && swizzle != 128)
-        return set_error(LENTILS_ERR_INVALID, "tma_map_bf16: swizzle %d", swizzle);
     if (rank < 1 || rank > 5 || !map || !base || ((uintptr_t)base & 15) != 0)
-        return set_error(LENTILS_ERR_INVALID, "tma_map_bf16: rank %d or unaligned base", rank);
-    if (box[0] * 2 > (uint32_t)swizzle)
-        return set_error(LENTILS_ERR_INVALID, "tma_map_bf16: inner box %u values", box[0]);
+        return set_error(LENTILS_ERR_INVALID, "tma_map: rank %d or unaligned base", rank);
     for (int i = 0; i + 1 < rank; ++i)
         if (strides[i] % 16 != 0)
-            return set_error(LENTILS_ERR_INVALID, "tma_map_bf16: stride %llu",
+            return set_error(LENTILS_ERR_INVALID, "tma_map: stride %llu",
                              (unsigned long long)strides[i]);
     PfnEncodeTiled enc;
     if (int st = encoder(&enc)) return st;
@@ -52,13 +49,30 @@ int tma_map_bf16(CUtensorMap *map, const void *base, int rank, const uint64_t *d
         es[i] = 1;
     }
     for (int i = 0; i + 1 < rank; ++i) gs[i] = strides[i];
-    const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank,
-                           const_cast<void *>(base), gd, gs, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           swizzle == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const CUresult r = enc(map, type, (cuuint32_t)rank, const_cast<void *>(base), gd, gs, bx, es,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error(LENTILS_ERR_CUDA, "cuTensorMapEncodeTiled: %d", (int)r);
     return LENTILS_OK;
+}
+
+int tma_map_bf16(CUtensorMap *map, const void *base, int rank, const uint64_t *dims,
+                 const uint64_t *strides, const uint32_t *box, int swizzle)
+{
+    if (swizzle != 64 && swizzle != 128)
+        return set_error(LENTILS_ERR_INVALID, "tma_map_bf16: swizzle %d", swizzle);
+    if (box[0] * 2 > (uint32_t)swizzle)
+        return set_error(LENTILS_ERR_INVALID, "tma_map_bf16: inner box %u values", box[0]);
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                  swizzle == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, base,
+                  rank, dims, strides, box);
+}
+
+int tma_map_f32(CUtensorMap *map, const void *base, int rank, const uint64_t *dims,
+                const uint64_t *strides, const uint32_t *box)
+{
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, CU_TENSOR_MAP_SWIZZLE_NONE, base, rank, dims,
+                  strides, box);
 }
 
 }  // namespace lentils

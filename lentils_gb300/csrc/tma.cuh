@@ -16,4 +16,8 @@ namespace lentils {
 int tma_map_bf16(CUtensorMap *map, const void *base, int rank, const uint64_t *dims,
                  const uint64_t *strides, const uint32_t *box, int swizzle = 128);
 
+// An FP32 tensor in the plain (unswizzled) layout, for TMA reductions.
+int tma_map_f32(CUtensorMap *map, const void *base, int rank, const uint64_t *dims,
+                const uint64_t *strides, const uint32_t *box);
+
 }  // namespace lentils

@@ -1964,6 +1964,284 @@ static int wgrad_mn_launch(const bf16 *x, const bf16 *dym, float *g, int C, int 
     return LENTILS_OK;
 }
 
+static int num_sms()
+{
+    static const int n = [] {
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            return 0;
+        return v;
+    }();
+    return n;
+}
+
+// CTA i of g takes rows [T i / g, T (i + 1) / g) of the T rows of a stack of images (or column
+// strips) of H rows: f(image, h0, h1) for each image's part, in order, until it returns false.
+template <class F>
+__device__ __forceinline__ void row_runs(int T, int H, int i, int g, F f)
+{
+    const int q1 = (int)((long long)T * (i + 1) / g);
+    for (int q = (int)((long long)T * i / g); q < q1;) {
+        const int n = q / H, h0 = q - n * H, h1 = min(H, h0 + (q1 - q));
+        if (!f(n, h0, h1)) return;
+        q += h1 - h0;
+    }
+}
+
+// Weight gradient of a 3 x 3 layer with row reuse. wgrad_mn_kernel loads each pixel of x once per
+// tap and of dym once per 128 rows of D (2.25 to 9 times), and that L2 -> SM traffic bounds it.
+// Here a CTA takes 32 input channels (blockIdx.x) and a run of image rows (blockIdx.y; strips of at
+// most 128 columns); it loads each row of dym once and each row of x once (one more at each end of
+// a run), with a column of padding on each side, into rings. One pixel is one 64-byte row of the
+// swizzled layout, whose chunk permutation goes by the address, so the horizontal taps are the same
+// slot 0, 64 and 128 bytes in: as the A operand's M atoms 64 bytes apart they make one MMA of
+// 128 rows (dx, ci), the fourth 32 of which (a fourth tap) are not read. Each of the three vertical
+// taps has its own N-column accumulator and reads the slot of its own row. The epilogue adds the
+// nine taps' blocks to g by TMA reductions. Warps and bounded waits as in wgrad_mn_kernel. Bound by
+// the latency of the row loads and the rate of the MN-major MMAs (about 100 clocks each).
+// Measured at batch 32, this kernel against wgrad_mn_kernel: 128 columns, 32 -> 32 channels
+// 27.6 / 50.2 us; 64 columns, 64 -> 32 21.6 / 29.6 and 32 -> 64 20.3 / 24.1; 32 columns, 64 -> 128
+// 21.8 / 27.5; 16 columns, 128 -> 128 34.7 / 11.6, which stays there.
+constexpr int kWgRowMax = 15;  // most rows of x in flight
+
+struct WgRowShape {
+    int wb;            // strip width
+    int xslot, dslot;  // bytes of a row's slot
+    int nx, nd;        // rows of x and of dym in flight: about 50 KB of x
+    int smem;
+};
+static WgRowShape wgrad_rows_shape(int N, int W)
+{
+    WgRowShape r;
+    r.wb = std::min(W, 128);
+    r.xslot = ((r.wb + 3) * 64 + 1023) / 1024 * 1024;  // the fourth tap reads one pixel more
+    r.dslot = (N / 32 * r.wb * 64 + 1023) / 1024 * 1024;
+    r.nx = 3 + 384 / r.wb;
+    r.nd = r.nx - 3;
+    const int ring = r.nx * r.xslot + r.nd * r.dslot, stage = 9 * N * 128;
+    r.smem = std::max(ring, stage) + 1024;
+    return r;
+}
+
+struct RingPos {  // slot l % n of a ring and the parity of its l-th use
+    int slot = 0, phase = 0;
+    __device__ __forceinline__ void next(int n)
+    {
+        if (++slot == n) {
+            slot = 0;
+            phase ^= 1;
+        }
+    }
+};
+
+template <int N>
+__global__ void __launch_bounds__(kWgMnThreads, 1)
+    wgrad_rows_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mdy,
+                      const __grid_constant__ CUtensorMap mg, int C, int H, int strips, int T,
+                      const WgRowShape sh, int *err)
+{
+    constexpr uint32_t ncols = 3 * N <= 128 ? 128 : 3 * N <= 256 ? 256 : 512;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    __shared__ uint64_t xfull[kWgRowMax], xempty[kWgRowMax], dfull[kWgRowMax], dempty[kWgRowMax], done;
+    __shared__ uint32_t tmem_base;
+    __shared__ int abort_flag;
+    unsigned char *xs = smem_raw + ((1024 - (tc::smem_u32(smem_raw) & 1023)) & 1023);
+    unsigned char *ds = xs + sh.nx * sh.xslot;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ci0 = blockIdx.x * 32, wb = sh.wb, nx = sh.nx, nd = sh.nd;
+    if (warp == 5) {
+        tc::tmem_alloc(&tmem_base, ncols);
+        tc::tmem_relinquish();
+    }
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < nx; ++i) {
+            tc::mbar_init(&xfull[i], 1);
+            tc::mbar_init(&xempty[i], 1);
+        }
+        for (int i = 0; i < nd; ++i) {
+            tc::mbar_init(&dfull[i], 1);
+            tc::mbar_init(&dempty[i], 1);
+        }
+        tc::mbar_init(&done, 1);
+        abort_flag = 0;
+        tc::fence_mbar_init();
+    }
+    if (threadIdx.x == 128) {
+        tc::prefetch_tensormap(&mx);
+        tc::prefetch_tensormap(&mdy);
+        tc::prefetch_tensormap(&mg);
+    }
+    tc::pdl_wait();
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    tc::pdl_trigger();
+    const uint32_t tmem = tmem_base;
+
+    if (warp == 4) {
+        if (lane == 0) {  // the TMA producer: x rows h0 - 1 .. h1, dym row h after x row h + 1
+            int lx = 0, ld = 0;
+            RingPos px, pd;
+            row_runs(T, H, blockIdx.y, gridDim.y, [&](int q, int h0, int h1) {
+                const int n = q / strips, w0 = (q - n * strips) * wb;
+                for (int r = h0 - 1; r <= h1; ++r) {
+                    if (lx >= nx && !tc::mbar_wait(&xempty[px.slot], px.phase ^ 1)) {
+                        atomicExch(&abort_flag, 1);
+                        return false;
+                    }
+                    tc::mbar_arrive_expect_tx(&xfull[px.slot], (uint32_t)(wb + 2) * 64u);
+                    tc::tma_load_4d(xs + px.slot * sh.xslot, &mx, ci0, w0 - 1, r, n, &xfull[px.slot]);
+                    ++lx;
+                    px.next(nx);
+                    if (r <= h0) continue;
+                    if (ld >= nd && !tc::mbar_wait(&dempty[pd.slot], pd.phase ^ 1)) {
+                        atomicExch(&abort_flag, 1);
+                        return false;
+                    }
+                    tc::mbar_arrive_expect_tx(&dfull[pd.slot], (uint32_t)wb * 2u * N);
+#pragma unroll
+                    for (int b = 0; b < N / 32; ++b)
+                        tc::tma_load_4d(ds + pd.slot * sh.dslot + b * wb * 64, &mdy, 32 * b, w0, r - 1,
+                                        n, &dfull[pd.slot]);
+                    ++ld;
+                    pd.next(nd);
+                }
+                return true;
+            });
+            // every load has landed before the CTA reuses shared memory or exits
+#pragma unroll 1
+            for (int i = 0; i < min(nx, lx); ++i)
+                if (!tc::mbar_wait(&xfull[i], ((lx - 1 - i) / nx) & 1)) atomicExch(&abort_flag, 1);
+#pragma unroll 1
+            for (int i = 0; i < min(nd, ld); ++i)
+                if (!tc::mbar_wait(&dfull[i], ((ld - 1 - i) / nd) & 1)) atomicExch(&abort_flag, 1);
+        }
+        __syncwarp();
+    } else if (warp == 5) {
+        if (lane == 0) {  // the MMA issuer
+            constexpr uint32_t idesc = tc::idesc_bf16_f32_mn(128, N);
+            const uint64_t da0 = tc::smem_desc_mn_sw64(tc::smem_u32(xs), 64, 512);
+            const uint64_t db0 = tc::smem_desc_mn_sw64(tc::smem_u32(ds), wb * 64, 512);
+            RingPos pl, pd;  // the next x row to wait for, the next dym row
+            int first = 0;   // slot of x row h - 1
+            uint32_t acc = 0;
+            bool ok = true;
+            row_runs(T, H, blockIdx.y, gridDim.y, [&](int, int h0, int h1) {
+                for (int h = h0 - 1; h <= h1; ++h) {
+                    if (!tc::mbar_wait(&xfull[pl.slot], pl.phase)) return ok = false;
+                    pl.next(nx);
+                    if (h <= h0) continue;  // rows h - 2 .. h: the output row h - 1
+                    if (!tc::mbar_wait(&dfull[pd.slot], pd.phase)) return ok = false;
+                    tc::tc_fence_after();
+                    const uint64_t b0 = tc::desc_step(db0, pd.slot * sh.dslot);
+                    int sl = first;
+#pragma unroll
+                    for (int dh = 0; dh < 3; ++dh) {
+                        uint64_t da = tc::desc_step(da0, sl * sh.xslot), db = b0;
+                        if (++sl == nx) sl = 0;
+                        tc::mma_bf16(tmem + dh * N, da, db, idesc, acc);
+#pragma unroll 7
+                        for (int k = 1; k < wb / 16; ++k) {
+                            da = tc::desc_step(da, 1024);
+                            db = tc::desc_step(db, 1024);
+                            tc::mma_bf16(tmem + dh * N, da, db, idesc, 1u);
+                        }
+                    }
+                    acc = 1;
+                    tc::mma_commit(&dempty[pd.slot]);
+                    pd.next(nd);
+                    tc::mma_commit(&xempty[first]);  // not read again
+                    if (++first == nx) first = 0;
+                }
+                for (int i = 0; i < 2; ++i) {
+                    tc::mma_commit(&xempty[first]);
+                    if (++first == nx) first = 0;
+                }
+                return true;
+            });
+            if (!ok) atomicExch(&abort_flag, 1);
+            tc::mma_commit(&done);
+        }
+        __syncwarp();
+    }
+    const bool fin = tc::mbar_wait(&done, 0);
+    tc::tc_fence_after();
+    __syncthreads();
+    const bool bad = !fin || *(volatile int *)&abort_flag;
+    if (threadIdx.x == 0 && bad) atomicExch(err, 1);
+    if (!bad && warp < 3) {  // warp = horizontal tap; N rows of 32 input channels per tap
+        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
+        float *stage = reinterpret_cast<float *>(xs) + warp * (32 * N);
+#pragma unroll 1
+        for (int dh = 0; dh < 3; ++dh, stage += 3 * 32 * N) {
+#pragma unroll 1
+            for (int n0 = 0; n0 < N; n0 += 32) {
+                uint32_t v[32];
+                tc::tmem_ld32(taddr + dh * N + n0, v);
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 32; ++i) stage[(n0 + i) * 32 + lane] = __uint_as_float(v[i]);
+            }
+            tc::fence_async_smem();
+            __syncwarp();
+            if (lane == 0) tc::tma_reduce_add_2d(&mg, (3 * dh + warp) * C + ci0, 0, stage);
+        }
+        if (lane == 0) tc::bulk_wait();
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 5) tc::tmem_dealloc(tmem, ncols);
+}
+
+// whether wgrad_rows_kernel takes a layer: 3 x 3, 32-channel boxes, whole MMA steps of 16 pixels
+// per strip row, and rows of at least 32 pixels (narrower ones are slower there than in
+// wgrad_mn_kernel; both figures above)
+static bool wgrad_rows_ok(int C, int N, int ks, int W)
+{
+    return ks == 3 && C % 32 == 0 && (N == 32 || N == 64 || N == 128) && W % 16 == 0 && W >= 32 &&
+           (W <= 128 || W % 128 == 0);
+}
+
+// Launches wgrad_rows_kernel (arguments as wgrad_mn_launch); ctas_want 0: as many CTAs as run at
+// once (by their accumulators: 512 columns of tensor memory per SM). A CTA adds 288 N values to
+// g, so it takes at least 512 pixels.
+template <int N>
+static int wgrad_rows_launch(const bf16 *x, const bf16 *dym, float *g, int C, int Bn, int H, int W,
+                             int ctas_want, int *err, cudaStream_t s)
+{
+    const WgRowShape sh = wgrad_rows_shape(N, W);
+    constexpr int kWgRowSmem = 200 * 1024;  // above every shape's
+    if (sh.nx > kWgRowMax || sh.smem > kWgRowSmem)
+        return set_error(LENTILS_ERR_UNSUPPORTED, "weight gradient rows: W=%d", W);
+    CUtensorMap mx, mdy;
+    const uint64_t dx[4] = {(uint64_t)C, (uint64_t)W, (uint64_t)H, (uint64_t)Bn};
+    const uint64_t sx[3] = {(uint64_t)C * 2, (uint64_t)W * C * 2, (uint64_t)H * W * C * 2};
+    const uint32_t bx[4] = {32, (uint32_t)sh.wb + 2, 1, 1};
+    if (int st = tma_map_bf16(&mx, x, 4, dx, sx, bx, 64)) return st;
+    const uint64_t dd[4] = {(uint64_t)N, (uint64_t)W, (uint64_t)H, (uint64_t)Bn};
+    const uint64_t sd[3] = {(uint64_t)N * 2, (uint64_t)W * N * 2, (uint64_t)H * W * N * 2};
+    const uint32_t bd[4] = {32, (uint32_t)sh.wb, 1, 1};
+    if (int st = tma_map_bf16(&mdy, dym, 4, dd, sd, bd, 64)) return st;
+    CUtensorMap mg;
+    const uint64_t dg[2] = {9 * (uint64_t)C, (uint64_t)N};
+    const uint64_t sg[1] = {9 * (uint64_t)C * 4};
+    const uint32_t bg[2] = {32, (uint32_t)N};
+    if (int st = tma_map_f32(&mg, g, 2, dg, sg, bg)) return st;
+    const int strips = W / sh.wb, T = Bn * strips * H, ncb = C / 32;
+    const int want = ctas_want > 0 ? ctas_want : std::max(1, num_sms()) * (N == 128 ? 1 : 2);
+    const long long px = (long long)Bn * H * W;
+    const int split = (int)std::max(1LL, std::min<long long>(std::min(T, std::max(1, want / ncb)), px / 512));
+    auto kern = wgrad_rows_kernel<N>;
+    static const cudaError_t attr = cudaFuncSetAttribute(
+        kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgRowSmem);
+    LENTILS_CUDA_TRY(attr);
+    LENTILS_CUDA_TRY(pdl_launch(kern, dim3(ncb, split), dim3(kWgMnThreads), (size_t)sh.smem, s, mx,
+                                mdy, mg, C, H, strips, T, sh, err));
+    LENTILS_CHECK_LAUNCH("weight gradient gemm (rows)");
+    return LENTILS_OK;
+}
+
 // whether wgrad_mn_kernel takes a layer: 32-channel boxes, 64-pixel chunks inside an image
 static bool wgrad_mn_ok(int C, int N, int H, int W)
 {
@@ -2041,18 +2319,6 @@ static int conv_tma_launch(const bf16 *act, int C, int ks, int Bn, int H, int W,
                                 K / 8, kp_per_split, err));
     LENTILS_CHECK_LAUNCH("convolution gemm (TMA)");
     return LENTILS_OK;
-}
-
-static int num_sms()
-{
-    static const int n = [] {
-        int dev = 0, v = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            return 0;
-        return v;
-    }();
-    return n;
 }
 
 // CTAs per SM of a persistent GEMM instantiation: as many as the SM's shared memory, registers
@@ -2187,19 +2453,6 @@ struct RowsSmem {
     static constexpr int kBytes = kB + kRowSlots * kSlot + 1024;
 };
 
-// CTA i of g takes rows [T i / g, T (i + 1) / g) of the T rows of a stack of images (or column
-// strips) of H rows: f(image, h0, h1) for each image's part, in order, until it returns false.
-template <class F>
-__device__ __forceinline__ void row_runs(int T, int H, int i, int g, F f)
-{
-    const int q1 = (int)((long long)T * (i + 1) / g);
-    for (int q = (int)((long long)T * i / g); q < q1;) {
-        const int n = q / H, h0 = q - n * H, h1 = min(H, h0 + (q1 - q));
-        if (!f(n, h0, h1)) return;
-        q += h1 - h0;
-    }
-}
-
 template <class EP>
 __global__ void __launch_bounds__(tc::kPersistThreads, 1)
     conv3_rows_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ CUtensorMap mb,
@@ -2279,40 +2532,45 @@ __global__ void __launch_bounds__(tc::kPersistThreads, 1)
             constexpr uint32_t idesc = tc::idesc_bf16_f32(128, 32);
             bool ok = tc::mbar_wait(&bfull, 0);
             tc::tc_fence_after();
-            int L = 0, j = 0;
+            const uint64_t dx = tc::smem_desc_sw64(tc::smem_u32(slots));
+            const uint64_t db = tc::smem_desc_sw64(tc::smem_u32(bres));
+            // tap (i, j) reads row i of three, j pixels into it; mirrored (flip) from the other end
+            const uint32_t w0 = flip ? 128 : 0;
+            const int dw = flip ? -64 : 64;
+            RingPos pl;     // the next row to wait for
+            int first = 0;  // slot of row h - 1
+            int j = 0;
             if (ok) row_runs(rows, H, blockIdx.x, gridDim.x, [&](int, int h0, int h1) {
-                const int nrows = h1 - h0 + 2;
-                int ready = 0;  // loads of this run known to have landed
-                for (int h = h0; h < h1; ++h, ++j) {
+                for (int r = h0 - 1; r <= h1; ++r) {
+                    if (!tc::mbar_wait(&sfull[pl.slot], pl.phase)) return ok = false;
+                    pl.next(S);
+                    if (r <= h0) continue;  // rows r - 2 .. r: the output row r - 1
                     const int buf = j & 1;
                     if (j >= 2 && !tc::mbar_wait(&tempty[buf], ((j >> 1) - 1) & 1)) return ok = false;
-                    for (; ready <= h - h0 + 2; ++ready) {
-                        const int Lr = L + ready;
-                        if (!tc::mbar_wait(&sfull[Lr % S], (Lr / S) & 1)) return ok = false;
-                    }
                     tc::tc_fence_after();
                     const uint32_t acc = tmem + (uint32_t)(buf * 32);
+                    const int mid = first + 1 == S ? 0 : first + 1, last = mid + 1 == S ? 0 : mid + 1;
 #pragma unroll
-                    for (int t = 0; t < 9; ++t) {
-                        int dh = t / 3 - 1, dw = t % 3 - 1;
-                        if (flip) {
-                            dh = -dh;
-                            dw = -dw;
-                        }
-                        const int Lr = L + (h + dh) - (h0 - 1);
-                        const uint32_t a = tc::smem_u32(slots + (Lr % S) * kSlot + (dw + 1) * 64);
-                        const uint32_t bb = tc::smem_u32(bres + t * 2048);
+                    for (int i = 0; i < 3; ++i) {
+                        const int sl = i == 1 ? mid : (i == 0) != (flip != 0) ? first : last;
+                        const uint64_t da = tc::desc_step(dx, sl * kSlot + w0);
 #pragma unroll
-                        for (int k = 0; k < 2; ++k)
-                            tc::mma_bf16(acc, tc::smem_desc_sw64(a + 32 * k), tc::smem_desc_sw64(bb + 32 * k),
-                                         idesc, (t > 0 || k > 0) ? 1u : 0u);
+                        for (int t = 3 * i; t < 3 * i + 3; ++t)
+#pragma unroll
+                            for (int k = 0; k < 2; ++k)
+                                tc::mma_bf16(acc, da + (uint64_t)((dw * (t - 3 * i) + 32 * k) / 16),
+                                             tc::desc_step(db, t * 2048 + 32 * k), idesc,
+                                             (t > 0 || k > 0) ? 1u : 0u);
                     }
                     tc::mma_commit(&tfull[buf]);
-                    tc::mma_commit(&sempty[(L + h - h0) % S]);  // row h - 1: no later tile reads it
+                    tc::mma_commit(&sempty[first]);  // no later tile reads it
+                    first = mid;
+                    ++j;
                 }
-                tc::mma_commit(&sempty[(L + nrows - 2) % S]);
-                tc::mma_commit(&sempty[(L + nrows - 1) % S]);
-                L += nrows;
+                for (int i = 0; i < 2; ++i) {
+                    tc::mma_commit(&sempty[first]);
+                    if (++first == S) first = 0;
+                }
                 return true;
             });
             if (!ok) atomicExch(&abort_flag, 1);
@@ -2616,7 +2874,11 @@ static int layer_backward(lentils_unet *net, int l, const bf16 *dy, const bf16 *
         int st = LENTILS_OK;
         if (mn) {
             const int ctas = net->wgrad_ctas > 0 ? net->wgrad_ctas : kWgradCtas;
-            switch (c.cout_p) {
+            if (wgrad_rows_ok(c.cin_p, c.cout_p, c.ks, W)) switch (c.cout_p) {
+            case 32: st = wgrad_rows_launch<32>(x, net->dym, net->gw_pad[l], c.cin_p, Bn, H, W, net->wgrad_ctas, net->err, s); break;
+            case 64: st = wgrad_rows_launch<64>(x, net->dym, net->gw_pad[l], c.cin_p, Bn, H, W, net->wgrad_ctas, net->err, s); break;
+            default: st = wgrad_rows_launch<128>(x, net->dym, net->gw_pad[l], c.cin_p, Bn, H, W, net->wgrad_ctas, net->err, s);
+            } else switch (c.cout_p) {
             case 32: st = wgrad_mn_launch<32>(x, net->dym, net->gw_pad[l], c.cin_p, c.ks, Bn, H, W, ctas, net->err, s); break;
             case 64: st = wgrad_mn_launch<64>(x, net->dym, net->gw_pad[l], c.cin_p, c.ks, Bn, H, W, ctas, net->err, s); break;
             case 128: st = wgrad_mn_launch<128>(x, net->dym, net->gw_pad[l], c.cin_p, c.ks, Bn, H, W, ctas, net->err, s); break;

@@ -280,3 +280,29 @@ def test_trained_network_in_flexible_cg(native):
                 (lrn, jac, plain)
         else:
             assert lrn["inner_total"] <= 2 * plain["inner_total"] + 50, (k, lrn, plain)
+
+
+@pytest.mark.parametrize("B,H,W", [(2, 16, 256), (3, 24, 64), (2, 40, 128), (1, 16, 32)])
+def test_weight_gradient_rows(native, B, H, W):
+    """The row form of the 3 x 3 weight gradients (two strips of 128 columns, rows of 128, 64 and 32
+    pixels) against the staged GEMMs, and with its pixel reduction in one run per channel block, in
+    runs that cut images anywhere, and as short as they come. The same inputs in another FP32 order:
+    at most 8192 products per sum, sqrt(8192) * 2^-24 = 5e-6 and twice that for both."""
+    from lentils_gb300 import _native as N
+    from lentils_gb300 import learned
+    p, x, f, t = _problem(31 + W, B, H, W)
+    net = learned.UNet(H, W, max_batch=B, params=p)
+    xc, fc, tc = _cuda(x, f, t)
+    g0, _ = net.gradients(xc, fc, tc)
+    for ctas in (1, 7, 60000):
+        N.check(N.lib().lentils_unet_set_wgrad_ctas(net.handle, ctas))
+        g, _ = net.gradients(xc, fc, tc)
+        assert _rel(g, g0) < 1e-5, (ctas, _rel(g, g0))
+    assert net.error_flag() == 0
+    net.set_gemm_form(1)
+    g1, _ = net.gradients(xc, fc, tc)
+    o = 0
+    for li, (ci, co, k, _, _) in enumerate(learned.LAYERS):
+        n = co * k * k * ci
+        assert _rel(g0[o:o + n], g1[o:o + n]) < 1e-2, li  # as test_unet_gemm_forms_agree
+        o += n + co
