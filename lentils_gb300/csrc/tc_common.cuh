@@ -109,6 +109,29 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
                  : "memory");
 }
 
+// -- clusters -------------------------------------------------------------------------------------
+// all threads of the cluster's CTAs; shared-memory writes before it are visible after it
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// the cluster-space address of this CTA's shared-memory address in the CTA of rank r
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t saddr, int r)
+{
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(r));
+    return a;
+}
+__device__ __forceinline__ float4 cluster_ld4(uint32_t addr)
+{
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(addr)
+                 : "memory");
+    return v;
+}
+
 // -- descriptors ----------------------------------------------------------------------------------
 // Shared-memory matrix descriptor: start address, LBO and SBO in 16-byte units, version 1,
 // no swizzle.

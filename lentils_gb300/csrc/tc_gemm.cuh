@@ -361,6 +361,21 @@ struct TmaSmem {
     static constexpr int kBytes = STAGES * kStageBytes + 1024;  // + alignment slack
 };
 
+// An epilogue with `static constexpr bool kCluster` finishes inside the kernel: the splits of a row
+// tile along K (gridDim.z of them) are one thread-block cluster, each leaves its FP32 partial tile
+// in its shared memory (rows of N + 4 values), and finish<N>() of every CTA works off its share of
+// the tile from all of them.
+template <class EP, class = void>
+struct cluster_epilogue {
+    static constexpr bool value = false;
+};
+template <class EP>
+struct cluster_epilogue<EP, decltype((void)EP::kCluster)> {
+    static constexpr bool value = EP::kCluster;
+};
+template <int N>
+constexpr int kClusterTileBytes = 128 * (N + 4) * 4 + 1024;
+
 template <int N, int STAGES, class LA, class LB, class EP>
 __global__ void __launch_bounds__(kPipeThreads)
     gemm_tma_kernel(const __grid_constant__ LA la, const __grid_constant__ LB lb, const EP ep,
@@ -460,7 +475,25 @@ __global__ void __launch_bounds__(kPipeThreads)
     __syncthreads();
     const bool bad = !fin || *(volatile int *)&abort_flag;
     if (threadIdx.x == 0 && bad) atomicExch(err, 1);
-    if (!bad && nchunks > 0 && warp < 4) {
+    if constexpr (cluster_epilogue<EP>::value) {
+        float *tile = reinterpret_cast<float *>(smem);
+        if (warp < 4) {
+            const int row = warp * 32 + (threadIdx.x & 31);
+            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
+#pragma unroll 4
+            for (int c0 = 0; c0 < N; c0 += 8) {
+                float v[8];
+                tmem_ld8(taddr + c0, v);
+                float4 *dst = reinterpret_cast<float4 *>(tile + row * (N + 4) + c0);
+                dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+                dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+            }
+        }
+        __syncwarp();
+        cluster_sync();
+        if (!bad) ep.template finish<N>(smem_u32(tile), m0, blockIdx.z, gridDim.z);
+        cluster_sync();  // no CTA leaves while another reads its tile
+    } else if (!bad && nchunks > 0 && warp < 4) {
         const int lane = threadIdx.x & 31;
         const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
         if constexpr (row_per_lane<EP>::value || N % 32 != 0) {

@@ -856,6 +856,99 @@ __global__ void finalize_up_kernel(const float *__restrict__ part, int nz,
     }
 }
 
+// finalize_pool_kernel and finalize_up_kernel as the epilogue of the split-K GEMM itself
+// (tc::gemm_tma_kernel, cluster form): the partial tiles are read from the shared memory of the
+// cluster's CTAs in the same order z = 0, 1, ..., so the values are the same bits, and a layer is
+// one launch instead of two. A tile of 128 pixels is 128 / W whole image rows, an even number of
+// them for pooling (W <= 64). Bound by latency: the U-Net of one 128^2 source 64.1 -> 60.6 us
+// (five kernels fewer).
+struct EpiClusterPost {
+    static constexpr bool kCluster = true;
+    bf16 *y;
+    const float *bias;
+    const bf16 *skip;  // null: pool
+    bf16 *post;
+    int W, relu;
+    // channels c .. c + 7 of pixel p of the tile
+    template <int N>
+    __device__ __forceinline__ void sum8(uint32_t tile, int p, int c, int nz, float (&v)[8]) const
+    {
+        const uint32_t o = tile + (uint32_t)(p * (N + 4) + c) * 4u;
+        float4 a[kSplitMax], b[kSplitMax];
+#pragma unroll
+        for (int z = 0; z < kSplitMax; ++z)
+            if (z < nz) {
+                const uint32_t r = tc::cluster_addr(o, z);
+                a[z] = tc::cluster_ld4(r);
+                b[z] = tc::cluster_ld4(r + 16);
+            }
+        v[0] = a[0].x, v[1] = a[0].y, v[2] = a[0].z, v[3] = a[0].w;
+        v[4] = b[0].x, v[5] = b[0].y, v[6] = b[0].z, v[7] = b[0].w;
+#pragma unroll
+        for (int z = 1; z < kSplitMax; ++z)
+            if (z < nz) {
+                v[0] += a[z].x, v[1] += a[z].y, v[2] += a[z].z, v[3] += a[z].w;
+                v[4] += b[z].x, v[5] += b[z].y, v[6] += b[z].z, v[7] += b[z].w;
+            }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            float t = v[i] + bias[c + i];
+            if (relu) t = fmaxf(t, 0.f);
+            v[i] = t;
+        }
+    }
+    template <int N>
+    __device__ __forceinline__ void finish(uint32_t tile, int m0, int rank, int nz) const
+    {
+        constexpr unsigned cv = N / 8, items = 128 * cv;  // whole warps
+        const unsigned step = nz * blockDim.x;
+        for (unsigned e = rank * blockDim.x + threadIdx.x; e < items; e += step) {
+            float v[8];
+            if (skip) {
+                const unsigned p = e / cv, c = (e % cv) * 8;
+                const unsigned q = m0 + p, r = q / W, w = q - r * W;  // row in the stack of images
+                float t[4][8];
+                size_t ph[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    ph[k] = ((size_t)(2 * r + (k >> 1)) * (2 * W) + 2 * w + (k & 1)) * N + c;
+                    bf8_load(skip + ph[k], t[k]);
+                }
+                sum8<N>(tile, p, c, nz, v);
+                bf8_store(y + (size_t)q * N + c, v);
+                float lo[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) lo[i] = bf(__float2bfloat16(v[i]));
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    float s[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) s[i] = lo[i] + t[k][i];
+                    bf8_store(post + ph[k], s);
+                }
+            } else {
+                const unsigned k = e & 3, rest = e >> 2, w2 = W / 2;
+                const unsigned q = rest / cv, c = (rest % cv) * 8;  // pooled pixel of the tile, channel
+                const unsigned r = q / w2, w = q - r * w2;
+                const unsigned p = (2 * r + (k >> 1)) * W + 2 * w + (k & 1);
+                sum8<N>(tile, p, c, nz, v);
+                bf8_store(y + (size_t)(m0 + p) * N + c, v);
+                float s[8];
+                const int src = threadIdx.x & 31 & ~3;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float yv = bf(__float2bfloat16(v[i]));  // the stored value, as pool2 reads it
+                    const float y1 = __shfl_sync(0xffffffffu, yv, src + 1);
+                    const float y2 = __shfl_sync(0xffffffffu, yv, src + 2);
+                    const float y3 = __shfl_sync(0xffffffffu, yv, src + 3);
+                    s[i] = 0.25f * (((yv + y1) + y2) + y3);
+                }
+                if (k == 0) bf8_store(post + (size_t)(m0 / 4 + q) * N + c, s);
+            }
+        }
+    }
+};
+
 // The pooling, upsampling and skip kernels and their adjoints move 16-byte groups of 8 channels; a
 // CTA walks image rows (of all images: row r of the stack of Bn H rows, whose low-resolution row
 // is r / 2), its threads the (pixel, channel group) pairs of a row, so the index arithmetic is
@@ -2310,13 +2403,19 @@ static int conv_tma_launch(const bf16 *act, int C, int ks, int Bn, int H, int W,
     const uint32_t bb[2] = {(uint32_t)CB, (uint32_t)N};
     if (int st = tma_map_bf16(&lb.map, wt, 2, db, sb, bb, 2 * CB)) return st;
     auto kern = tc::gemm_tma_kernel<N, kStages, ConvTmaA<CB>, ConvTmaB<CB, N>, EP>;
-    constexpr int smem = tc::TmaSmem<N, kStages, CB>::kBytes;
+    constexpr bool cluster = tc::cluster_epilogue<EP>::value;
+    constexpr int smem = cluster ? std::max(tc::TmaSmem<N, kStages, CB>::kBytes, tc::kClusterTileBytes<N>)
+                                 : tc::TmaSmem<N, kStages, CB>::kBytes;
     static const cudaError_t attr =
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     LENTILS_CUDA_TRY(attr);
     const int mtiles = Bn * H * W / 128;
-    LENTILS_CUDA_TRY(pdl_launch(kern, dim3(mtiles, 1, nz), dim3(tc::kPipeThreads), smem, s, la, lb, ep,
-                                K / 8, kp_per_split, err));
+    if constexpr (cluster)
+        LENTILS_CUDA_TRY(pdl_launch_cluster(kern, dim3(mtiles, 1, nz), dim3(tc::kPipeThreads), smem, s,
+                                            dim3(1, 1, nz), la, lb, ep, K / 8, kp_per_split, err));
+    else
+        LENTILS_CUDA_TRY(pdl_launch(kern, dim3(mtiles, 1, nz), dim3(tc::kPipeThreads), smem, s, la, lb,
+                                    ep, K / 8, kp_per_split, err));
     LENTILS_CHECK_LAUNCH("convolution gemm (TMA)");
     return LENTILS_OK;
 }
@@ -2768,6 +2867,12 @@ static int layer_forward(lentils_unet *net, int l, const bf16 *x, void *y, int B
     const int nz = (kp + per - 1) / per;
     const long long n = (long long)npix * c.cout_p;
     if (npix < kSplitMaxPix && nz > 1 && nz * n <= (long long)kSplitSlabPix * 128) {
+        // form 0: summed inside the GEMM, with the post step (whole pooling blocks per tile)
+        if (persist && (post.up || (post.pool && W <= 64))) {
+            const EpiClusterPost ep{(bf16 *)y, net->b32[l], post.up ? post.skip : nullptr,
+                                    post.up ? post.up : post.pool, W, c.relu};
+            return conv_tma(x, c.cin_p, c.ks, Bn, H, W, 0, net->wf[l], c.cout_p, ep, nz, per, net->err, s);
+        }
         EpiPartialF32 ep{net->splitk, npix, c.cout_p};
         int st = LENTILS_OK;
         if (tma) st = conv_tma(x, c.cin_p, c.ks, Bn, H, W, 0, net->wf[l], c.cout_p, ep, nz, per, net->err, s);

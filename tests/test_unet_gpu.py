@@ -306,3 +306,22 @@ def test_weight_gradient_rows(native, B, H, W):
         n = co * k * k * ci
         assert _rel(g0[o:o + n], g1[o:o + n]) < 1e-2, li  # as test_unet_gemm_forms_agree
         o += n + co
+
+
+@pytest.mark.parametrize("B,H,W", [(1, 64, 64), (1, 32, 64), (1, 256, 64), (2, 16, 32), (1, 128, 256),
+                                   (1, 16, 128), (3, 64, 16)])
+def test_split_layers_finish_in_clusters(native, B, H, W):
+    """Split layers whose partial tiles are summed inside a thread-block cluster, with pooling or
+    upsampling (2 to 8 splits; tiles of 1, 2, 4 and 8 image rows and of whole small images; rows too
+    wide to pool in a tile), against the staged GEMMs: as test_unet_gemm_forms_agree."""
+    from lentils_gb300 import learned
+    p, x, f, t = _problem(13 + W, B, H, W)
+    net = learned.UNet(H, W, max_batch=B, params=p)
+    xc, fc = _cuda(x, f)
+    out = [net.forward(xc, fc).cpu().numpy() for _ in range(2)]
+    assert np.array_equal(out[0], out[1])
+    net.set_gemm_form(1)
+    ref = net.forward(xc, fc).cpu().numpy()
+    assert net.error_flag() == 0
+    assert _rel(out[0], ref) < 2e-3
+    assert np.max(np.abs(out[0] - ref)) < 0.02 * np.max(np.abs(ref))
