@@ -33,10 +33,10 @@ constexpr int kDeflectThreads = 128;
 // A thread takes NP pairs of neighbouring points, blockDim.x pairs apart (packed arithmetic, one
 // point per half). Bound by instruction issue; the lens constants of a launch come through the
 // constant cache by an index, so each costs an instruction to fetch and one to pair, which NP = 2
-// spreads over four points. 1.7e7 FP32 points, PEMD + shear + two multipole orders: 116 us
-// (2.3 TB/s of points; 348 us with one point per thread, complex square root, powf, atan2f and
-// sincosf); NP = 1 takes 137 us. The packed FMA pipe is 67 % busy. VEC (FP32 points on 16-byte aligned arrays): a pair is one 16-byte
-// load and store.
+// spreads over four points. 1.7e7 FP32 points, PEMD + shear + two multipole orders: 128 us
+// (2.1 TB/s of points; 348 us with one point per thread, complex square root, powf, atan2f and
+// sincosf); NP = 1 takes about 20 us more. The packed FMA pipe is two thirds busy. VEC (FP32
+// points on 16-byte aligned arrays): a pair is one 16-byte load and store.
 template <typename P, bool VEC, int NP>
 __global__ void __launch_bounds__(kDeflectThreads, NP == 2 ? 6 : 1)
     deflect_kernel(const P *pin, P *pout, long long n, const __grid_constant__ DevLensSet lenses,
@@ -214,7 +214,7 @@ static int deflect_launch(const lentils_mass_model *lenses, int nlenses, const P
         return set_error(LENTILS_ERR_INVALID, "deflect: bad arguments");
     if (n == 0) return LENTILS_OK;
     // four points per thread once that still gives every SM four CTAs (1.7e7 points: 116 us
-    // against 137 us with two); below that the second pair would only leave SMs idle
+    // against 137 us with two, measured before the constants' low parts were added); below that the second pair would only leave SMs idle
     const bool four = n >= 152LL * 2048;
     const long long per = (four ? 4 : 2) * kDeflectThreads;
     const int blocks = (int)std::min<long long>((n + per - 1) / per, 152LL * 128);

@@ -2377,6 +2377,25 @@ static int wgrad_launch(const ConvWgXT &la, const ConvWgDyT &lb, const EpiAtomic
     return LENTILS_OK;
 }
 
+constexpr int conv_tma_stages(int CB, int N) { return CB == 64 && N == 128 ? 3 : 4; }
+
+template <int CB, int N, class EP>
+constexpr int conv_tma_smem()
+{
+    constexpr int ring = tc::TmaSmem<N, conv_tma_stages(CB, N), CB>::kBytes;
+    return tc::cluster_epilogue<EP>::value ? std::max(ring, tc::kClusterTileBytes<N>) : ring;
+}
+
+// the shared-memory limit of one instantiation (set once per process)
+template <int CB, int N, class EP>
+static cudaError_t conv_tma_attr()
+{
+    static const cudaError_t attr = cudaFuncSetAttribute(
+        tc::gemm_tma_kernel<N, conv_tma_stages(CB, N), ConvTmaA<CB>, ConvTmaB<CB, N>, EP>,
+        cudaFuncAttributeMaxDynamicSharedMemorySize, conv_tma_smem<CB, N, EP>());
+    return attr;
+}
+
 // A convolution GEMM with TMA operands: activations act (NHWC, C channels, Bn images of
 // H x W; flip: data gradient), weights wt (row-major [N][K], K = ks^2 C), rows = pixels,
 // split over nz CTAs of kp_per_split pieces along K.
@@ -2385,7 +2404,7 @@ static int conv_tma_launch(const bf16 *act, int C, int ks, int Bn, int H, int W,
                            const bf16 *wt, int K, const EP &ep, int nz, int kp_per_split,
                            int *err, cudaStream_t s)
 {
-    constexpr int kStages = (CB == 64 && N == 128) ? 3 : 4;
+    constexpr int kStages = conv_tma_stages(CB, N);
     ConvTmaA<CB> la;
     la.C = C;
     la.ks = ks;
@@ -2404,11 +2423,8 @@ static int conv_tma_launch(const bf16 *act, int C, int ks, int Bn, int H, int W,
     if (int st = tma_map_bf16(&lb.map, wt, 2, db, sb, bb, 2 * CB)) return st;
     auto kern = tc::gemm_tma_kernel<N, kStages, ConvTmaA<CB>, ConvTmaB<CB, N>, EP>;
     constexpr bool cluster = tc::cluster_epilogue<EP>::value;
-    constexpr int smem = cluster ? std::max(tc::TmaSmem<N, kStages, CB>::kBytes, tc::kClusterTileBytes<N>)
-                                 : tc::TmaSmem<N, kStages, CB>::kBytes;
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    LENTILS_CUDA_TRY(attr);
+    constexpr int smem = conv_tma_smem<CB, N, EP>();
+    LENTILS_CUDA_TRY((conv_tma_attr<CB, N, EP>()));
     const int mtiles = Bn * H * W / 128;
     if constexpr (cluster)
         LENTILS_CUDA_TRY(pdl_launch_cluster(kern, dim3(mtiles, 1, nz), dim3(tc::kPipeThreads), smem, s,
@@ -3366,6 +3382,11 @@ static int prepare_forward()
     LENTILS_CUDA_TRY((gemm_smem_attr<32, ConvFwdA, tc::RowMajorLoader, EpiPartialF32>()));
     LENTILS_CUDA_TRY((gemm_smem_attr<64, ConvFwdA, tc::RowMajorLoader, EpiPartialF32>()));
     LENTILS_CUDA_TRY((gemm_smem_attr<128, ConvFwdA, tc::RowMajorLoader, EpiPartialF32>()));
+    LENTILS_CUDA_TRY((conv_tma_attr<32, 32, EpiClusterPost>()));
+    LENTILS_CUDA_TRY((conv_tma_attr<32, 64, EpiClusterPost>()));
+    LENTILS_CUDA_TRY((conv_tma_attr<64, 32, EpiClusterPost>()));
+    LENTILS_CUDA_TRY((conv_tma_attr<64, 64, EpiClusterPost>()));
+    LENTILS_CUDA_TRY((conv_tma_attr<64, 128, EpiClusterPost>()));
     LENTILS_CUDA_TRY((conv_persist_shape<32, 32, RowAct>().err));
     LENTILS_CUDA_TRY((conv_persist_shape<32, 64, RowAct>().err));
     LENTILS_CUDA_TRY((conv_persist_shape<32, 128, RowAct>().err));
