@@ -33,8 +33,8 @@ constexpr int kDeflectThreads = 128;
 // A thread takes NP pairs of neighbouring points, blockDim.x pairs apart (packed arithmetic, one
 // point per half). Bound by instruction issue; the lens constants of a launch come through the
 // constant cache by an index, so each costs an instruction to fetch and one to pair, which NP = 2
-// spreads over four points. 1.7e7 FP32 points, PEMD + shear + two multipole orders: 128 us
-// (2.1 TB/s of points; 348 us with one point per thread, complex square root, powf, atan2f and
+// spreads over four points. 1.7e7 FP32 points, PEMD + shear + two multipole orders: 123 us
+// (2.2 TB/s of points; 348 us with one point per thread, complex square root, powf, atan2f and
 // sincosf); NP = 1 takes about 20 us more. The packed FMA pipe is two thirds busy. VEC (FP32
 // points on 16-byte aligned arrays): a pair is one 16-byte load and store.
 template <typename P, bool VEC, int NP>
@@ -162,7 +162,7 @@ int build_lens(const lentils_mass_model &m, DevLens &L)
         const double n = hypot((double)L.cth, (double)L.sth) / hypot(p[4], p[5]);
         const double amp = b * b / q * pow(b, t - 2.0) / pow(n, 2.0 - t);
         L.amp = (float)amp;
-        L.amp1 = L.amp != 0.f ? (float)((amp - (double)L.amp) / (double)L.amp) : 0.f;
+        L.ampl = isfinite(L.amp) ? (float)(amp - (double)L.amp) : 0.f;
         set_power(L, 0.5 * (2.0 - t));
         double an = 1.0;
         for (int n = 0; n < kSeriesTerms; ++n) {
@@ -214,7 +214,7 @@ static int deflect_launch(const lentils_mass_model *lenses, int nlenses, const P
         return set_error(LENTILS_ERR_INVALID, "deflect: bad arguments");
     if (n == 0) return LENTILS_OK;
     // four points per thread once that still gives every SM four CTAs (1.7e7 points: 116 us
-    // against 137 us with two, measured before the constants' low parts were added); below that the second pair would only leave SMs idle
+    // against 137 us with two; 123 now with their constants' low parts); below that the second pair would only leave SMs idle
     const bool four = n >= 152LL * 2048;
     const long long per = (four ? 4 : 2) * kDeflectThreads;
     const int blocks = (int)std::min<long long>((n + per - 1) / per, 152LL * 128);

@@ -18,10 +18,10 @@ struct DevLens {
     double x0, y0;
     float x0h, x0l, y0h, y0l;  // the centre as FP32 pairs: x0 = x0h + x0l to ~2^-48 relative
     float gxh, gxl, gyh, gyl;  // batched sweep: its sample's pixel-grid origin minus the centre
-    // PEMD: alpha = conj(amp (1 + amp1) * rs2^h * F(u) * rot / z), see pemd_setup. The second
-    // parts hold what FP32 drops of amp and q^2: a rounding of a constant moves every point the
-    // same way, where the roundings of the points' own values average out.
-    float cth, sth, q2, q2l, cx, cy, amp, amp1;
+    // PEMD: alpha = conj((amp + ampl) * rs2^h * F(u) * rot / z), see pemd_setup. The second parts
+    // hold what FP32 drops of amp and q^2: a rounding of a constant moves every point the same
+    // way, where the roundings of the points' own values average out.
+    float cth, sth, q2, q2l, cx, cy, amp, ampl;
     int nterms;   // series terms (kSeriesTerms: the full series, complex Horner)
     int tail;     // some points have |u| >= 0.75
     float an[kSeriesTerms];
@@ -215,8 +215,9 @@ static __device__ __forceinline__ float2 series_tail(const DevLens &L, double dx
 // without a complex square root, and |u| <= max(|cx|, |cy|) at every point: the number of
 // series terms that FP32 can tell apart follows from q alone (build_lens). The prefactor
 // b'^2 / (q z) (b' / r_s)^(t - 2) is amp (r_s^2)^h / z, h = (2 - t) / 2, amp = b'^t / q.
-// One reciprocal, of |z|^2, serves both quotients. Gives z, u and a = amp (1 + amp1)
-// (r_s^2)^h / |z|^2.
+// One reciprocal, of |z|^2, serves both quotients. Gives z, u and a = (amp + ampl)
+// (r_s^2)^h / |z|^2. The low parts of amp and q^2 enter by products that are rounded once together
+// with the high ones: added to a product rounded before, they would be below half its last place.
 __device__ __forceinline__ void pemd_setup(const DevLens &L, float2 dx, float2 dy, float2 ct,
                                            float2 st, float2 ns, float2 &X, float2 &Y,
                                            float2 &ur, float2 &ui, float2 &a)
@@ -224,13 +225,12 @@ __device__ __forceinline__ void pemd_setup(const DevLens &L, float2 dx, float2 d
     X = __ffma2_rn(dx, ct, __fmul2_rn(dy, st));  // z = (dx + i dy) (cth - i sth)
     Y = __ffma2_rn(dy, ct, __fmul2_rn(dx, ns));
     const float2 xx = __fmul2_rn(X, X), yy = __fmul2_rn(Y, Y), xy = __fmul2_rn(X, Y);
-    const float2 rs2 = __ffma2_rn(splat(L.q2l), xx, __ffma2_rn(splat(L.q2), xx, yy));
+    const float2 rs2 = __fadd2_rn(__ffma2_rn(splat(L.q2), xx, __fmul2_rn(splat(L.q2l), xx)), yy);
     const float2 pw = lens_power(L, rs2);
     const float2 inv = recip2(__fadd2_rn(xx, yy));
     ur = __fmul2_rn(__ffma2_rn(splat(L.cx), xx, __fmul2_rn(splat(L.cy), yy)), inv);
     ui = __fmul2_rn(__fmul2_rn(splat(L.cy - L.cx), xy), inv);
-    const float2 a0 = __fmul2_rn(__fmul2_rn(splat(L.amp), pw), inv);
-    a = __ffma2_rn(a0, splat(L.amp1), a0);
+    a = __fmul2_rn(__ffma2_rn(splat(L.amp), pw, __fmul2_rn(splat(L.ampl), pw)), inv);
 }
 
 __device__ __forceinline__ void shear_alpha(const DevLens &L, float sx, float sy, float &ax,
