@@ -57,3 +57,44 @@ def test_convolution(native, nx, ny):
     assert O.rel_l2(op * x, ref) < 1e-14
     got = op * torch.as_tensor(x, dtype=torch.float32).cuda()
     assert O.rel_l2(got.cpu().numpy(), ref) < 5.7e-7
+
+
+@pytest.mark.parametrize("real,cplx,tol", [(torch.float32, torch.complex64, 1.2e-6),
+                                           (torch.float64, torch.complex128, 3e-12)])
+def test_adjoint_leaves_its_grid_zero(native, real, cplx, tol):
+    """The adjoint accumulates into a grid that its own column transform leaves zero: repeated, with
+    forward calls between, and captured and replayed, each call gives the adjoint of its own input.
+    Tolerances as above."""
+    from lentils_gb300.operators import NUFFTOperator
+    from lentils_gb300.spaces import ImageSpace, VisibilitySpace
+    rng = np.random.default_rng(12)
+    n, b = 64, [(-0.5, 0.3), (-0.2, 0.9)]
+    img = O.ImageGeom((n, n), b)
+    padded, _, _ = O.padded_geom(img, 2)
+    uvw = O.synth_uv(rng, 1500, O.FourierGeom(padded), 0.45, 4)
+    ora = O.NufftOracle(O.VisGeom(uvw, [1.0]), img, 2, 4)
+    op = NUFFTOperator(VisibilitySpace([1.0], uvw), ImageSpace((n, n), b), 2, 4)
+    xs = [rng.normal(size=(n, n)) for _ in range(2)]
+    ref = [ora.adjoint(ora.forward(x)).reshape(n, n) for x in xs]
+    ys = [(op * torch.as_tensor(x).cuda()).to(cplx) for x in xs]
+
+    def check(got, i):
+        assert O.rel_l2(got.cpu().numpy(), ref[i]) < tol
+    for i in (0, 1, 1, 0):
+        check(op.T * ys[i], i)
+        op * torch.as_tensor(xs[1 - i], dtype=real).cuda()
+    static = ys[0].clone()
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(s):
+        op.T * static
+        torch.cuda.synchronize()
+        with torch.cuda.graph(g, stream=s):
+            out = op.T * static
+    torch.cuda.current_stream().wait_stream(s)
+    for i in (0, 1, 0):
+        static.copy_(ys[i])
+        g.replay()
+        check(out, i)
+        check(op.T * ys[1 - i], 1 - i)
