@@ -214,7 +214,8 @@ static int deflect_launch(const lentils_mass_model *lenses, int nlenses, const P
         return set_error(LENTILS_ERR_INVALID, "deflect: bad arguments");
     if (n == 0) return LENTILS_OK;
     // four points per thread once that still gives every SM four CTAs (1.7e7 points: 116 us
-    // against 137 us with two; 123 now with their constants' low parts); below that the second pair would only leave SMs idle
+    // against 137 us with two; 123 us now, with the constants' low parts); below that the second
+    // pair would only leave SMs idle
     const bool four = n >= 152LL * 2048;
     const long long per = (four ? 4 : 2) * kDeflectThreads;
     const int blocks = (int)std::min<long long>((n + per - 1) / per, 152LL * 128);
