@@ -140,9 +140,11 @@ static int bcb_init(lentils_bcb *op, const double *beam, cudaStream_t s)
     LENTILS_CUDA_TRY(cudaMalloc(&op->real32, sizeof(float) * nr));
     op->own = fft2d_supported(op->px, op->py);
     if (op->own) {
-        int st = fft2d_init<float2>(&op->fft32, op->nx, op->ny, op->padx, op->pady, op->px, op->py);
+        int st = fft2d_init<float2>(&op->fft32, op->nx, op->ny, op->padx, op->pady, op->px, op->py,
+                                    s);
         if (!st)
-            st = fft2d_init<double2>(&op->fft64, op->nx, op->ny, op->padx, op->pady, op->px, op->py);
+            st = fft2d_init<double2>(&op->fft64, op->nx, op->ny, op->padx, op->pady, op->px,
+                                     op->py, s);
         if (st) return st;
     } else {
         LENTILS_CUDA_TRY(cudaMalloc(&op->work64, sizeof(double2) * nc));

@@ -651,7 +651,8 @@ int lentils_normal_op_create(lentils_normal_op **out, lentils_lensop *L, lentils
         }
         op->wsum = sum;
         if (e == cudaSuccess)
-            e = cudaMemcpy(op->w32, hf.data(), sizeof(float) * nvis, cudaMemcpyHostToDevice);
+            e = cudaMemcpyAsync(op->w32, hf.data(), sizeof(float) * nvis, cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
             const int st = cuda_status(e, "normal_op_create weights");
             normal_op_free(op);
@@ -988,7 +989,8 @@ int lentils_fcg_solve(lentils_normal_op *op, const double *b, double *x, const f
         FCGWindow hw;
         memset(&hw, 0, sizeof(hw));
         hw.m = m;
-        e = cudaMemcpy(win, &hw, sizeof(hw), cudaMemcpyHostToDevice);
+        e = cudaMemcpyAsync(win, &hw, sizeof(hw), cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     }
     if (e != cudaSuccess) st = cuda_status(e, "fcg_solve alloc");
     if (!st && net) st = lentils_unet_features(inv_diag32, feat, n, stream);

@@ -430,7 +430,7 @@ bool fft2d_supported(int nu, int nv) { return fft_size(nu) && fft_size(nv); }
 
 // Twiddles of passes 2 and 3 (q Ns + k: exp(-2 pi i k q / (Ns R))); pass 3's start at 16 R2.
 template <typename C>
-static int upload_twiddles(int n, void **dst)
+static int upload_twiddles(int n, void **dst, cudaStream_t s)
 {
     const int r2 = n >= 256 ? 16 : n / 16, r3 = n / (16 * r2);
     std::vector<C> h(16 * r2 + (r3 > 1 ? n : 0));
@@ -445,19 +445,20 @@ static int upload_twiddles(int n, void **dst)
         for (int q = 0; q < r3; ++q)
             for (int k = 0; k < 16 * r2; ++k) set(h[16 * r2 + q * 16 * r2 + k], k, q, n);
     LENTILS_CUDA_TRY(cudaMalloc(dst, sizeof(C) * h.size()));
-    LENTILS_CUDA_TRY(cudaMemcpy(*dst, h.data(), sizeof(C) * h.size(), cudaMemcpyHostToDevice));
+    LENTILS_CUDA_TRY(cudaMemcpyAsync(*dst, h.data(), sizeof(C) * h.size(), cudaMemcpyHostToDevice, s));
+    LENTILS_CUDA_TRY(cudaStreamSynchronize(s));
     return LENTILS_OK;
 }
 
 template <typename C>
-int fft2d_init(Fft2d *op, int nx, int ny, int padx, int pady, int nu, int nv)
+int fft2d_init(Fft2d *op, int nx, int ny, int padx, int pady, int nu, int nv, cudaStream_t s)
 {
     *op = Fft2d{nx, ny, padx, pady, nu, nv, nv / 2 + 1, fft2d_pitch(nv), nullptr, nullptr};
-    if (int st = upload_twiddles<C>(nu, &op->tw_u)) return st;
-    return upload_twiddles<C>(nv, &op->tw_v);
+    if (int st = upload_twiddles<C>(nu, &op->tw_u, s)) return st;
+    return upload_twiddles<C>(nv, &op->tw_v, s);
 }
-template int fft2d_init<float2>(Fft2d *, int, int, int, int, int, int);
-template int fft2d_init<double2>(Fft2d *, int, int, int, int, int, int);
+template int fft2d_init<float2>(Fft2d *, int, int, int, int, int, int, cudaStream_t);
+template int fft2d_init<double2>(Fft2d *, int, int, int, int, int, int, cudaStream_t);
 
 void fft2d_free(Fft2d *op)
 {

@@ -20,9 +20,10 @@ struct Fft2d {
     void *tw_u, *tw_v;       // twiddle tables (device), float2 or double2
 };
 
-// Twiddle tables of `op` in FP32 (C = float2) or FP64 (double2); free them with fft2d_free.
+// Twiddle tables of `op` in FP32 (C = float2) or FP64 (double2), uploaded on s and complete on
+// return; free them with fft2d_free.
 template <typename C>
-int fft2d_init(Fft2d *op, int nx, int ny, int padx, int pady, int nu, int nv);
+int fft2d_init(Fft2d *op, int nx, int ny, int padx, int pady, int nu, int nv, cudaStream_t s);
 void fft2d_free(Fft2d *op);
 
 // Image -> half-plane spectrum (nu x half) of the zero-padded image, unnormalised. apx (nx) and

@@ -195,6 +195,7 @@ int lentils_nufft_create(lentils_nufft **out, const lentils_plan *plan, int nx, 
     op->nv = plan->geom.nv;
     op->half_nv = plan->geom.half_nv;
     op->precisions = precisions;
+    cudaStream_t s = (cudaStream_t)stream;
     const size_t ngrid = (size_t)op->nu * op->half_nv;
     const size_t npad = std::max((size_t)op->nu * op->nv, 2 * (size_t)nx * fft2d_pitch(op->nv));
     op->own = fft2d_supported(op->nu, op->nv);
@@ -207,6 +208,13 @@ int lentils_nufft_create(lentils_nufft **out, const lentils_plan *plan, int nx, 
         delete op;
         return set_error(c ? c : code, "%s", msg);
     };
+    // on the caller's stream and complete on return: a copy from pageable memory on the legacy
+    // stream need not have landed when it returns, and nothing orders it before kernels on a
+    // non-blocking stream
+    auto upload = [&](auto *dst, const auto *src, int n) {
+        const cudaError_t c = cudaMemcpyAsync(dst, src, sizeof(*src) * n, cudaMemcpyHostToDevice, s);
+        return c == cudaSuccess ? cudaStreamSynchronize(s) : c;
+    };
     cudaError_t e = cudaSuccess;
     if (precisions & 1) {
         e = cudaMalloc(&op->apx32, sizeof(float) * nx);
@@ -217,21 +225,20 @@ int lentils_nufft_create(lentils_nufft **out, const lentils_plan *plan, int nx, 
             std::vector<float> fx(nx), fy(ny);
             for (int i = 0; i < nx; ++i) fx[i] = (float)apod_x[i];
             for (int j = 0; j < ny; ++j) fy[j] = (float)apod_y[j];
-            e = cudaMemcpy(op->apx32, fx.data(), sizeof(float) * nx, cudaMemcpyHostToDevice);
-            if (e == cudaSuccess)
-                e = cudaMemcpy(op->apy32, fy.data(), sizeof(float) * ny, cudaMemcpyHostToDevice);
+            e = upload(op->apx32, fx.data(), nx);
+            if (e == cudaSuccess) e = upload(op->apy32, fy.data(), ny);
         }
         if (e != cudaSuccess) {
             cuda_status(e, "nufft_create (FP32 buffers)");
             return fail(LENTILS_ERR_CUDA);
         }
         if (op->own) {
-            if (fft2d_init<float2>(&op->fft32, nx, ny, padx, pady, op->nu, op->nv))
+            if (fft2d_init<float2>(&op->fft32, nx, ny, padx, pady, op->nu, op->nv, s))
                 return fail(LENTILS_ERR_CUDA);
             e = cudaMalloc(&op->acc32, sizeof(float2) * ngrid);
             if (e == cudaSuccess)
-                e = cudaMemsetAsync(op->acc32, 0, sizeof(float2) * ngrid, (cudaStream_t)stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
+                e = cudaMemsetAsync(op->acc32, 0, sizeof(float2) * ngrid, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
             if (e != cudaSuccess) {
                 cuda_status(e, "nufft_create (FP32 buffers)");
                 return fail(LENTILS_ERR_CUDA);
@@ -251,21 +258,19 @@ int lentils_nufft_create(lentils_nufft **out, const lentils_plan *plan, int nx, 
         if (e == cudaSuccess) e = cudaMalloc(&op->apy64, sizeof(double) * ny);
         if (e == cudaSuccess) e = cudaMalloc(&op->pad64, sizeof(double) * npad);
         if (e == cudaSuccess) e = cudaMalloc(&op->grid64, sizeof(double2) * ngrid);
-        if (e == cudaSuccess)
-            e = cudaMemcpy(op->apx64, apod_x, sizeof(double) * nx, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess)
-            e = cudaMemcpy(op->apy64, apod_y, sizeof(double) * ny, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = upload(op->apx64, apod_x, nx);
+        if (e == cudaSuccess) e = upload(op->apy64, apod_y, ny);
         if (e != cudaSuccess) {
             cuda_status(e, "nufft_create (FP64 buffers)");
             return fail(LENTILS_ERR_CUDA);
         }
         if (op->own) {
-            if (fft2d_init<double2>(&op->fft64, nx, ny, padx, pady, op->nu, op->nv))
+            if (fft2d_init<double2>(&op->fft64, nx, ny, padx, pady, op->nu, op->nv, s))
                 return fail(LENTILS_ERR_CUDA);
             e = cudaMalloc(&op->acc64, sizeof(double2) * ngrid);
             if (e == cudaSuccess)
-                e = cudaMemsetAsync(op->acc64, 0, sizeof(double2) * ngrid, (cudaStream_t)stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize((cudaStream_t)stream);
+                e = cudaMemsetAsync(op->acc64, 0, sizeof(double2) * ngrid, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
             if (e != cudaSuccess) {
                 cuda_status(e, "nufft_create (FP64 buffers)");
                 return fail(LENTILS_ERR_CUDA);

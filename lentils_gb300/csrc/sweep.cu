@@ -553,18 +553,20 @@ int lentils_sweep_create(lentils_sweep **out, const lentils_sweep_sample *in, in
     if (e == cudaSuccess && !hl.empty())
         e = cudaMemcpyAsync(sw->lenses, hl.data(), sizeof(DevLens) * hl.size(), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = sweep_set_smem(sw->form, (int)sw->smem);
+    std::vector<std::vector<SweepItem>> hgroups(sw->groups.size());
+    std::vector<int2> hchunk;  // sources of copies on s, as hs, hw and hl: until the wait below
     if (sw->split) {
         const auto longest = [](const auto &x, const auto &y) { return x.first > y.first; };
         for (size_t q = 0; q < sw->groups.size() && e == cudaSuccess; ++q) {
             SweepGroup &g = sw->groups[q];
             std::stable_sort(gitems[q].begin(), gitems[q].end(), longest);
-            std::vector<SweepItem> h;
+            std::vector<SweepItem> &h = hgroups[q];
             for (const auto &x : gitems[q]) h.push_back(x.second);
             g.nitems = (int)h.size();
             e = cudaMalloc(&g.items, sizeof(SweepItem) * std::max<size_t>(1, h.size()));
             if (e == cudaSuccess && !h.empty())
-                e = cudaMemcpy(g.items, h.data(), sizeof(SweepItem) * h.size(),
-                               cudaMemcpyHostToDevice);
+                e = cudaMemcpyAsync(g.items, h.data(), sizeof(SweepItem) * h.size(),
+                                    cudaMemcpyHostToDevice, s);
             if (e == cudaSuccess)
                 e = g.w2 == 8 ? sweep_smem_attr(sweep_grid_kernel<8>)
                               : sweep_smem_attr(sweep_grid_kernel<6>);
@@ -573,12 +575,13 @@ int lentils_sweep_create(lentils_sweep **out, const lentils_sweep_sample *in, in
                               : sweep_smem_attr(sweep_degrid_kernel<6>);
         }
         std::stable_sort(chunks.begin(), chunks.end(), longest);
-        std::vector<int2> h;
-        for (const auto &x : chunks) h.push_back(x.second);
-        sw->nchunks = (int)h.size();
-        if (e == cudaSuccess) e = cudaMalloc(&sw->chunks, sizeof(int2) * std::max<size_t>(1, h.size()));
-        if (e == cudaSuccess && !h.empty())
-            e = cudaMemcpy(sw->chunks, h.data(), sizeof(int2) * h.size(), cudaMemcpyHostToDevice);
+        for (const auto &x : chunks) hchunk.push_back(x.second);
+        sw->nchunks = (int)hchunk.size();
+        if (e == cudaSuccess)
+            e = cudaMalloc(&sw->chunks, sizeof(int2) * std::max<size_t>(1, hchunk.size()));
+        if (e == cudaSuccess && !hchunk.empty())
+            e = cudaMemcpyAsync(sw->chunks, hchunk.data(), sizeof(int2) * hchunk.size(),
+                                cudaMemcpyHostToDevice, s);
         for (int k = 0; k < 2 && e == cudaSuccess; ++k) {
             e = cudaStreamCreateWithFlags(&sw->side[k], cudaStreamNonBlocking);
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sw->join[k], cudaEventDisableTiming);
