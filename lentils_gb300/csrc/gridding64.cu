@@ -11,8 +11,8 @@
 //         half. Six packed instructions per complex tap (a sum without bias takes eleven: the
 //         product's own rounding and Knuth's two-sum).
 // The bias follows the data: in degridding the largest value of each row of the visibility's own
-// window, in gridding the sums so far and the largest of the next 2w visibilities, so the
-// rounding is relative to values that reach the same results.
+// window, in gridding the sums so far and the largest of the next visibilities of the same cell,
+// so the rounding is relative to values that reach the same results.
 // The weights are fits of degree 11 here (9 in the FP64 kernels, which differ from the profile
 // by 1.1e-10 of its peak at w = 4): within 1e-12 of the peak, so that the pairs' rounding does
 // not add to the fit's error but takes its place. F^T F of a 512^2 image with 2e6 visibilities
@@ -392,12 +392,13 @@ __global__ void __launch_bounds__(kDsThreads, 3)
     const int rbeg = min(it.count, gid * L), rend = lane_on ? min(it.count, rbeg + L) : rbeg;
     const int nbatch = (L + W2 - 1) / W2;
     const unsigned gmask = ((1u << W2) - 1u) << (grp * W2);
-    // the lanes of this lane's group; those beyond the last group form one of their own
-    const unsigned gmask_all = lane_on ? gmask : ~0u << (G * W2 % 32);
     float *rowg = rows + gid * Row::GSTR;
     float *myrow = rowg + ri * Row::STR;
 
-    // acc[j].h carries the bias B[j]; |term| <= row_peak * kb.peak[j] * |x|
+    // acc[j].h carries the bias B[j]; |term| <= row_peak * kb.peak[j] * |x|. A batch of sorted
+    // visibilities may span several cells, so the bias is chosen for each run of one cell, from
+    // that run's own |x|: a strong visibility must not set the rounding of cells that it does not
+    // reach. (Figures at the kernel.)
     const float row_peak = (float)W2 * kb.peak[ri];
     float B[W2];
     DS acc[W2];
@@ -406,7 +407,9 @@ __global__ void __launch_bounds__(kDsThreads, 3)
         B[j] = bias(0);
         acc[j] = DS{f2(B[j]), f2(0.f)};
     }
-    auto flush_to = [&](int cell) {
+    // xr: largest biased exponent of the run that the sums are for next
+    auto flush_to = [&](int cell, int xr) {
+        const float rx = row_peak * __int_as_float((xr + 1) << 23);
         float4 *p = mytile + ((cell >> 6) + 1 + ri) * S + (cell & 63) + 1;
 #pragma unroll
         for (int j = 0; j < W2; ++j) {
@@ -414,6 +417,7 @@ __global__ void __launch_bounds__(kDsThreads, 3)
             acc[j].h = __fadd2_rn(acc[j].h, f2(-B[j]));
             const DS r = ds_add(DS{make_float2(f.x, f.y), make_float2(f.z, f.w)}, acc[j]);
             p[j] = make_float4(r.h.x, r.h.y, r.l.x, r.l.y);
+            B[j] = bias((__float_as_int(rx * kb.peak[j]) >> 23) - 125);
             acc[j] = DS{f2(B[j]), f2(0.f)};
         }
     };
@@ -490,12 +494,24 @@ __global__ void __launch_bounds__(kDsThreads, 3)
         wm &= (1u << W2) - 1u;
         const unsigned bm = lane_on ? (flags >> (grp * W2)) & ((1u << W2) - 1u) : 0u;
         const int steps = (int)(lane_on ? nvalid : 0);
-        // Renormalise the sums and choose each tap's bias for this batch: above its sum so far
-        // plus 2w terms of the batch's largest |x| and the taps' largest weights. (Without this
-        // the low halves would grow past the last place of the high ones.)
-        xe = __reduce_max_sync(gmask_all, xe);
+        // the largest |x| of this lane's run from here on (equal cells are neighbours; lanes of
+        // the next group with the same cell may count too)
+#pragma unroll
+        for (int d = 1; d < W2; d <<= 1) {
+            const int ke = __shfl_down_sync(0xffffffffu, key, d);
+            const int xo = __shfl_down_sync(0xffffffffu, xe, d);
+            if (ke == key) xe = max(xe, xo);
+        }
+        // Renormalise the sums and choose each tap's bias for what this batch adds to them: above
+        // the sum so far plus 2w terms of the largest |x| of the batch's first run, if that is of
+        // the sums' cell, and the taps' largest weights. (Without this the low halves would grow
+        // past the last place of the high ones.)
         {
-            const float rx = row_peak * __int_as_float((xe + 1) << 23);
+            const int k0 = __shfl_sync(0xffffffffu, key, grp * W2);
+            const int x0 = __shfl_sync(0xffffffffu, xe, grp * W2);
+            const float rx = cell0 < 0 || k0 == cell0
+                                 ? row_peak * __int_as_float((x0 + 1) << 23)
+                                 : 0.f;
 #pragma unroll
             for (int j = 0; j < W2; ++j) {
                 const float2 v = __fadd2_rn(acc[j].h, f2(-B[j]));  // exact
@@ -519,10 +535,11 @@ __global__ void __launch_bounds__(kDsThreads, 3)
                 const bool need = (bm >> st) & 1u;
                 const int before = __shfl_sync(0xffffffffu, key, grp * W2 + max(st, 1) - 1);
                 const int fcell = st > 0 ? before : cell0;
+                const int xr = __shfl_sync(0xffffffffu, xe, grp * W2 + st);
                 unsigned gm = __ballot_sync(0xffffffffu, need);
                 while (gm) {
                     const int g0 = (__ffs(gm) - 1) / W2;
-                    if (need && grp == g0) flush_to(fcell);
+                    if (need && grp == g0) flush_to(fcell, xr);
                     __syncwarp();
                     gm &= ~(((1u << W2) - 1u) << (g0 * W2));
                 }
@@ -558,7 +575,7 @@ __global__ void __launch_bounds__(kDsThreads, 3)
     }
 #pragma unroll 1
     for (int g0 = 0; g0 < G; ++g0) {
-        if (lane_on && grp == g0 && plast >= 0) flush_to(plast);
+        if (lane_on && grp == g0 && plast >= 0) flush_to(plast, 0);
         __syncwarp();
     }
     __syncthreads();
