@@ -10,9 +10,10 @@
 //         the product's remainder; that and the cross terms wh gl + wl gh collect in the low
 //         half. Six packed instructions per complex tap (a sum without bias takes eleven: the
 //         product's own rounding and Knuth's two-sum).
-// The bias follows the data: in degridding the largest value of each row of the visibility's own
-// window, in gridding the sums so far and the largest of the next visibilities of the same cell,
-// so the rounding is relative to values that reach the same results.
+// The bias follows the data, the real and the imaginary part each: in degridding the largest value
+// of each row of the visibility's own window, in gridding the sums so far and the largest of the
+// next visibilities of the same cell, so the rounding is relative to values that reach the same
+// results.
 // The weights are fits of degree 11 here (9 in the FP64 kernels, which differ from the profile
 // by 1.1e-10 of its peak at w = 4): within 1e-12 of the peak, so that the pairs' rounding does
 // not add to the fit's error but takes its place. F^T F of a 512^2 image with 2e6 visibilities
@@ -21,9 +22,10 @@
 //
 // Range. FP32 exponents do not cover FP64's, so a work item scales its tile (degrid) or its
 // visibilities (grid) by the power of two that brings the largest finite one to [1, 2) and the
-// result back. A value keeps all 48 bits down to 2^-78 of that largest value, and is zero below
-// 2^-126 of it. Infinities and NaN go through as such: where the high half of a result is not
-// finite it is the result.
+// result back. A value keeps all 48 bits down to 2^-77 of that largest value. What lies below it
+// (far(): subnormals too) does not go through pairs: a tile with such a value is degridded in
+// FP64, and such a visibility is added to the grid in FP64, with the same weights. Infinities and
+// NaN go through as such: where the high half of a result is not finite it is the result.
 #include <algorithm>
 #include <cmath>
 
@@ -51,10 +53,27 @@ __device__ __forceinline__ void ds_mac(float wh, float wl, const DS &g, DS &r)
     r.h = s;
 }
 
-// 1.5 * 2^m for partial sums below 2^(m - 1)
-__device__ __forceinline__ float bias(int m)
+// The bias 1.5 * 2^m with 2^(m - 1) above |bound|, per part.
+__device__ __forceinline__ float bias(float bound)
 {
-    return __int_as_float(((m + 127) << 23) | 0x400000);
+    return __int_as_float((((__float_as_int(bound) >> 23) + 2) << 23) | 0x400000);
+}
+__device__ __forceinline__ float2 bias(float2 bound)
+{
+    return make_float2(bias(bound.x), bias(bound.y));
+}
+
+// Biased exponents of the real and the imaginary part, in the halves of a word (maxima by
+// __vmaxu2), and the powers of two above the values of such exponents. The parts are separate sums:
+// each has its own bias.
+__device__ __forceinline__ unsigned exponents(int re, int im)
+{
+    return (unsigned)re | (unsigned)im << 16;
+}
+__device__ __forceinline__ float2 above(unsigned e)
+{
+    return make_float2(__int_as_float((int)((e & 0xffff) + 1) << 23),
+                       __int_as_float((int)((e >> 16) + 1) << 23));
 }
 
 __device__ __forceinline__ bool finite(float v) { return fabsf(v) <= 3.402823466e38f; }
@@ -134,6 +153,13 @@ __device__ __forceinline__ int exponent_of(double v)  // biased; 0 for zero, sub
     return e == 0x7ff ? 0 : e;
 }
 
+// whether v is too small beside a value of biased exponent emax for a pair to hold its bits
+__device__ __forceinline__ bool far(double v, int emax)
+{
+    const int e = (__double2hiint(v) >> 20) & 0x7ff;
+    return e < max(1, emax - 77) && v != 0.0;
+}
+
 // v * 2^(1023 - emax) as h + l (emax: biased exponent of the largest value, at least 1)
 __device__ __forceinline__ void split(double v, int emax, float &h, float &l)
 {
@@ -182,6 +208,79 @@ __device__ __forceinline__ int block_max_exponent(int e, int *red)
 
 constexpr int kDsThreads = 128;
 
+// Cell (ea, eb) of the extended tile at (a0, b0), through the Hermitian fold.
+__device__ __forceinline__ double2 tile_cell(const double2 *__restrict__ grid, const GridGeom &g,
+                                             int a0, int b0, int ea, int eb)
+{
+    int au = wrap_index(a0 + ea, g.nu), bv = wrap_index(b0 + eb, g.nv);
+    const bool conj = bv >= g.half_nv;
+    if (conj) {
+        au = (g.nu - au) % g.nu;
+        bv = g.nv - bv;
+    }
+    double2 v = grid[(long long)au * g.half_nv + bv];
+    if (conj) v.y = -v.y;
+    return v;
+}
+
+// The item of degrid_ds_kernel in FP64, with the same weights: tiles whose values span more than
+// the pairs' range. Rare, and not inlined, so that the paired path keeps its registers.
+template <int W2>
+static __device__ __noinline__ void degrid_far(const double2 *__restrict__ grid,
+                                               const uint2 *__restrict__ coords,
+                                               const float2 *__restrict__ cres,
+                                               double2 *__restrict__ out,
+                                               const WorkItem *__restrict__ items,
+                                               const KBPolyDS &kb, const GridGeom &g,
+                                               const double *__restrict__ vscale,
+                                               unsigned char *smraw)
+{
+    constexpr int w = W2 / 2;
+    double2 *sm = reinterpret_cast<double2 *>(smraw);  // as many bytes as the pairs
+    const WorkItem it = items[blockIdx.x];
+    const int a0 = it.tu * g.T - g.Hu - w, b0 = it.tv * g.T - g.Hv - w, E = g.E, S = g.stride;
+    for (int e = threadIdx.x; e < E * E; e += kDsThreads)
+        sm[e / E * S + e % E] = tile_cell(grid, g, a0, b0, e / E, e % E);
+    __syncthreads();
+    for (int k = threadIdx.x; k < it.count; k += kDsThreads) {
+        const uint2 c = coords[it.begin + k];
+        const float2 rr = cres[it.begin + k];
+        const int lu = cell_of(c.x), lv = cell_of(c.y);
+        float uh[W2], ul[W2], vh[W2], vl[W2];
+        ds_weights<W2>(kb, c.y, rr.y, vh, vl);
+        ds_weights<W2>(kb, c.x, rr.x, uh, ul);
+        double wv[W2], re = 0.0, im = 0.0;  // wv with scale2: subnormal cells keep their bits
+#pragma unroll
+        for (int j = 0; j < W2; ++j) wv[j] = ((double)vh[j] + (double)vl[j]) * kb.scale2;
+        auto row = [&](double wu, const double2 *p) {
+            double tr = 0.0, ti = 0.0;
+#pragma unroll
+            for (int j = 0; j < W2; ++j) {
+                tr = fma(wv[j], p[j].x, tr);
+                ti = fma(wv[j], p[j].y, ti);
+            }
+            re = fma(wu, tr, re);
+            im = fma(wu, ti, im);
+        };
+        const double2 *p = sm + (lu + 1) * S + (lv + 1);
+#pragma unroll
+        for (int i = 0; i < W2; ++i) row((double)uh[i] + (double)ul[i], p + i * S);
+        if (c.x & kExtraTapBit) row(kb.edge, p - S);
+        if (c.y & kExtraTapBit) {
+            auto column = [&](double wu, const double2 &q) {
+                re = fma(wu * kb.edge * kb.scale2, q.x, re);
+                im = fma(wu * kb.edge * kb.scale2, q.y, im);
+            };
+#pragma unroll
+            for (int i = 0; i < W2; ++i) column((double)uh[i] + (double)ul[i], p[i * S - 1]);
+            if (c.x & kExtraTapBit) column(kb.edge, p[-S - 1]);
+        }
+        double sc = tap_parity(it, g, lu, lv) ? -1.0 : 1.0;
+        if (vscale) sc *= vscale[it.begin + k];
+        out[it.begin + k] = make_double2(re * sc, im * sc);
+    }
+}
+
 // Degridding: one visibility per thread over the staged tile (as degrid_item). Bound by the
 // FP32 pipe: about 450 packed instructions for the taps and 630 for the weights of a
 // visibility.
@@ -190,56 +289,50 @@ __global__ void __launch_bounds__(kDsThreads, W2 == 6 ? 3 : 4)  // 4 would spill
     degrid_ds_kernel(const double2 *__restrict__ grid, const uint2 *__restrict__ coords,
                      const float2 *__restrict__ cres, double2 *__restrict__ out,
                      const WorkItem *__restrict__ items, const __grid_constant__ KBPolyDS kb,
-                     const GridGeom g, const double *__restrict__ vscale)
+                     const __grid_constant__ GridGeom g, const double *__restrict__ vscale)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     float4 *sm = reinterpret_cast<float4 *>(smraw);  // (h.re, h.im, l.re, l.im) per cell
-    // largest exponent (biased) of the 2w cells of a row that a cell's window covers
-    unsigned char *rowmax = reinterpret_cast<unsigned char *>(sm + g.E * g.stride);  // E x T
+    // largest exponents (biased; real, imaginary) of the 2w cells of a row that a cell's window
+    // covers, E x T
+    uchar2 *rowmax = reinterpret_cast<uchar2 *>(sm + g.E * g.stride);
     __shared__ int red[kDsThreads / 32];
     constexpr int w = W2 / 2;
     pdl_entry();
     const WorkItem it = items[blockIdx.x];
     const int a0 = it.tu * g.T - g.Hu - w, b0 = it.tv * g.T - g.Hv - w;
     const int E = g.E, S = g.stride;
-    auto fetch = [&](int ea, int eb, bool &conj) {
-        int au = wrap_index(a0 + ea, g.nu), bv = wrap_index(b0 + eb, g.nv);
-        conj = bv >= g.half_nv;
-        if (conj) {
-            au = (g.nu - au) % g.nu;
-            bv = g.nv - bv;
-        }
-        return grid[(long long)au * g.half_nv + bv];
-    };
     int emax = 0;
     for (int e = threadIdx.x; e < E * E; e += kDsThreads) {
-        bool conj;
-        const double2 v = fetch(e / E, e % E, conj);
+        const double2 v = tile_cell(grid, g, a0, b0, e / E, e % E);
         emax = max(emax, max(exponent_of(v.x), exponent_of(v.y)));
     }
     emax = block_max_exponent(emax, red);
+    bool out_of_range = false;
     for (int e = threadIdx.x; e < E * E; e += kDsThreads) {
         const int ea = e / E, eb = e - ea * E;
-        bool conj;
-        double2 v = fetch(ea, eb, conj);
-        if (conj) v.y = -v.y;
+        const double2 v = tile_cell(grid, g, a0, b0, ea, eb);
+        out_of_range |= far(v.x, emax) || far(v.y, emax);
         float4 q;
         split(v.x, emax, q.x, q.z);
         split(v.y, emax, q.y, q.w);
         sm[ea * S + eb] = q;
     }
-    __syncthreads();
-    auto exponent = [](const float4 &q) {  // of a cell; 0 where it is not finite
+    if (__syncthreads_or(out_of_range)) {
+        degrid_far<W2>(grid, coords, cres, out, items, kb, g, vscale, smraw);
+        return;
+    }
+    auto of_cell = [](const float4 &q) {  // 0 where a part is not finite
         const int a = (__float_as_int(q.x) >> 23) & 0xff, b = (__float_as_int(q.y) >> 23) & 0xff;
-        return max(a == 0xff ? 0 : a, b == 0xff ? 0 : b);
+        return exponents(a == 0xff ? 0 : a, b == 0xff ? 0 : b);
     };
     const int T = g.T;
     for (int e = threadIdx.x; e < E * T; e += kDsThreads) {
         const int ea = e / T, lv = e - ea * T;
-        int m = 0;
+        unsigned m = 0;
 #pragma unroll
-        for (int j = 0; j < W2; ++j) m = max(m, exponent(sm[ea * S + lv + 1 + j]));
-        rowmax[e] = (unsigned char)m;
+        for (int j = 0; j < W2; ++j) m = __vmaxu2(m, of_cell(sm[ea * S + lv + 1 + j]));
+        rowmax[e] = make_uchar2(m & 0xff, m >> 16);
     }
     __syncthreads();
     const int es = emax - 1023;
@@ -254,26 +347,27 @@ __global__ void __launch_bounds__(kDsThreads, W2 == 6 ? 3 : 4)  // 4 would spill
         const float4 *p = sm + (lu + 1) * S + (lv + 1);
         // the cells of a window row are below 2^(e - 126) and the v-weights sum to less than 1;
         // the window's sum is below the sum of the rows' bounds times the u-weights
-        const unsigned char *rm = rowmax + (lu + 1) * T + lv;
-        float bound = 0.f;
+        const uchar2 *rm = rowmax + (lu + 1) * T + lv;
+        auto row_above = [&](int i) { return above(exponents(rm[i * T].x, rm[i * T].y)); };
+        float2 bound = f2(0.f);
 #pragma unroll
-        for (int i = 0; i < W2; ++i)
-            bound = fmaf(fabsf(uh[i]), __int_as_float(((int)rm[i * T] + 1) << 23), bound);
-        const float BA = bias((__float_as_int(bound) >> 23) - 125);
-        DS acc{f2(BA), f2(0.f)};
+        for (int i = 0; i < W2; ++i) bound = __ffma2_rn(f2(fabsf(uh[i])), row_above(i), bound);
+        const float2 BA = bias(bound);
+        DS acc{BA, f2(0.f)};
 #pragma unroll
         for (int i = 0; i < W2; ++i) {
-            const float B = bias((int)rm[i * T] - 125);
-            DS r{f2(B), f2(0.f)};
+            // (a row's bound is a power of two: half of it has the bias that its exponent asks for)
+            const float2 B = bias(__fmul2_rn(f2(0.5f), row_above(i)));
+            DS r{B, f2(0.f)};
 #pragma unroll
             for (int j = 0; j < W2; ++j) {
                 const float4 q = p[i * S + j];
                 ds_mac(vh[j], vl[j], DS{make_float2(q.x, q.y), make_float2(q.z, q.w)}, r);
             }
-            r.h = __fadd2_rn(r.h, f2(-B));
+            r.h = minus(r.h, B);
             ds_mac(uh[i], ul[i], r, acc);
         }
-        acc.h = __fadd2_rn(acc.h, f2(-BA));
+        acc.h = minus(acc.h, BA);
         double re, im;
         if ((c.x | c.y) & kExtraTapBit) {
             // the taps at argument +w, in FP64 (coordinates on a cell boundary only)
@@ -368,6 +462,7 @@ __global__ void __launch_bounds__(kDsThreads, 3)
     emax = block_max_exponent(emax, red);
     const int es = emax - 1023 - 1;  // with the factor 1/2 of the gridding
     const double s1 = pow2(es / 2), s2 = pow2(es - es / 2) * kb.scale2;
+    const double unscaled = 0.5 * kb.scale2;  // the same for values that are not scaled
     const int a0 = it.tu * g.T - g.Hu - w, b0 = it.tv * g.T - g.Hv - w;
     auto to_grid = [&](int ea, int eb, double re, double im) {
         int au = wrap_index(a0 + ea, g.nu), bv = wrap_index(b0 + eb, g.nv);
@@ -398,27 +493,27 @@ __global__ void __launch_bounds__(kDsThreads, 3)
     // acc[j].h carries the bias B[j]; |term| <= row_peak * kb.peak[j] * |x|. A batch of sorted
     // visibilities may span several cells, so the bias is chosen for each run of one cell, from
     // that run's own |x|: a strong visibility must not set the rounding of cells that it does not
-    // reach. (Figures at the kernel.)
+    // reach. (F^T F of 2e6 visibilities, w = 4: 579 us, and 582 with one bias per batch.)
     const float row_peak = (float)W2 * kb.peak[ri];
-    float B[W2];
+    float2 B[W2];
     DS acc[W2];
 #pragma unroll
     for (int j = 0; j < W2; ++j) {
-        B[j] = bias(0);
-        acc[j] = DS{f2(B[j]), f2(0.f)};
+        B[j] = bias(f2(0.f));
+        acc[j] = DS{B[j], f2(0.f)};
     }
-    // xr: largest biased exponent of the run that the sums are for next
-    auto flush_to = [&](int cell, int xr) {
-        const float rx = row_peak * __int_as_float((xr + 1) << 23);
+    // xr: largest biased exponents of the run that the sums are for next
+    auto flush_to = [&](int cell, unsigned xr) {
+        const float2 rx = __fmul2_rn(f2(row_peak), above(xr));
         float4 *p = mytile + ((cell >> 6) + 1 + ri) * S + (cell & 63) + 1;
 #pragma unroll
         for (int j = 0; j < W2; ++j) {
             const float4 f = p[j];
-            acc[j].h = __fadd2_rn(acc[j].h, f2(-B[j]));
+            acc[j].h = minus(acc[j].h, B[j]);
             const DS r = ds_add(DS{make_float2(f.x, f.y), make_float2(f.z, f.w)}, acc[j]);
             p[j] = make_float4(r.h.x, r.h.y, r.l.x, r.l.y);
-            B[j] = bias((__float_as_int(rx * kb.peak[j]) >> 23) - 125);
-            acc[j] = DS{f2(B[j]), f2(0.f)};
+            B[j] = bias(__fmul2_rn(rx, f2(kb.peak[j])));
+            acc[j] = DS{B[j], f2(0.f)};
         }
     };
     int plast = -1;  // cell of the group's sums, -1: none
@@ -426,17 +521,28 @@ __global__ void __launch_bounds__(kDsThreads, 3)
         __syncwarp();
         const int kv = rbeg + b * W2 + ri;
         const bool valid = kv < rend;
-        int key = -1, xe = 0;
+        int key = -1;
+        unsigned xe = 0;
+        double2 fx = make_double2(0.0, 0.0);  // parts beyond the pairs' range
         if (valid) {
             const uint2 c = coords[it.begin + kv];
             const float2 rr = cres[it.begin + kv];
             const double2 x = vis[it.begin + kv];
-            xe = max(0, max(exponent_of(x.x), exponent_of(x.y)) - emax + 127);
+            xe = exponents(max(0, exponent_of(x.x) - emax + 127),
+                           max(0, exponent_of(x.y) - emax + 127));
             const int lu = cell_of(c.x), lv = cell_of(c.y);
             const float sg = tap_parity(it, g, lu, lv) ? -1.f : 1.f;
             float4 xs;
             split(x.x, emax, xs.x, xs.z);
             split(x.y, emax, xs.y, xs.w);
+            if (far(x.x, emax)) {
+                fx.x = sg * unscaled * x.x;
+                xs.x = xs.z = 0.f;
+            }
+            if (far(x.y, emax)) {
+                fx.y = sg * unscaled * x.y;
+                xs.y = xs.w = 0.f;
+            }
             key = (lu << 6) | lv;
             float4 *r4 = reinterpret_cast<float4 *>(myrow);
             r4[Row::X / 4] = make_float4(sg * xs.x, sg * xs.y, sg * xs.z, sg * xs.w);
@@ -466,11 +572,8 @@ __global__ void __launch_bounds__(kDsThreads, 3)
                 // to the grid
                 const double eu = (c.x & kExtraTapBit) ? kb.edge : 0.0;
                 const double ev = (c.y & kExtraTapBit) ? kb.edge : 0.0;
-                const double xr = sg * ((double)xs.x + (double)xs.z);
-                const double xi = sg * ((double)xs.y + (double)xs.w);
-                auto put = [&](int ea, int eb, double wt) {
-                    to_grid(ea, eb, wt * xr * s1 * s2, wt * xi * s1 * s2);
-                };
+                const double xr = sg * unscaled * x.x, xi = sg * unscaled * x.y;
+                auto put = [&](int ea, int eb, double wt) { to_grid(ea, eb, wt * xr, wt * xi); };
                 if (eu != 0.0) {
                     for (int j = 0; j < W2; ++j)
                         put(lu, lv + 1 + j, eu * ((double)vh[j] + (double)vl[j]));
@@ -479,6 +582,21 @@ __global__ void __launch_bounds__(kDsThreads, 3)
                 if (ev != 0.0)
                     for (int i = 0; i < W2; ++i)
                         put(lu + 1 + i, lv, ev * ((double)uh[i] + (double)ul[i]));
+            }
+        }
+        // visibilities beyond the range: in FP64, straight to the grid, the taps over the lanes
+        for (unsigned fm = __ballot_sync(0xffffffffu, fx.x != 0.0 || fx.y != 0.0); fm;
+             fm &= fm - 1) {
+            const int src = __ffs(fm) - 1;
+            const double xr = __shfl_sync(0xffffffffu, fx.x, src);
+            const double xi = __shfl_sync(0xffffffffu, fx.y, src);
+            const int cell = __shfl_sync(0xffffffffu, key, src);
+            const float *row = rows + (warp * G + src / W2) * Row::GSTR + (src % W2) * Row::STR;
+            for (int e = lane; e < W2 * W2; e += 32) {
+                const int i = e / W2, j = e % W2;
+                const double wt = ((double)row[Row::U + 2 * i] + (double)row[Row::U + 2 * i + 1]) *
+                                  ((double)row[j] + (double)row[Row::WP + j]);
+                to_grid((cell >> 6) + 1 + i, (cell & 63) + 1 + j, wt * xr, wt * xi);
             }
         }
         const int up = __shfl_up_sync(0xffffffffu, key, 1);
@@ -499,8 +617,8 @@ __global__ void __launch_bounds__(kDsThreads, 3)
 #pragma unroll
         for (int d = 1; d < W2; d <<= 1) {
             const int ke = __shfl_down_sync(0xffffffffu, key, d);
-            const int xo = __shfl_down_sync(0xffffffffu, xe, d);
-            if (ke == key) xe = max(xe, xo);
+            const unsigned xo = __shfl_down_sync(0xffffffffu, xe, d);
+            if (ke == key) xe = __vmaxu2(xe, xo);
         }
         // Renormalise the sums and choose each tap's bias for what this batch adds to them: above
         // the sum so far plus 2w terms of the largest |x| of the batch's first run, if that is of
@@ -508,23 +626,18 @@ __global__ void __launch_bounds__(kDsThreads, 3)
         // past the last place of the high ones.)
         {
             const int k0 = __shfl_sync(0xffffffffu, key, grp * W2);
-            const int x0 = __shfl_sync(0xffffffffu, xe, grp * W2);
-            const float rx = cell0 < 0 || k0 == cell0
-                                 ? row_peak * __int_as_float((x0 + 1) << 23)
-                                 : 0.f;
+            const unsigned x0 = __shfl_sync(0xffffffffu, xe, grp * W2);
+            const float2 rx = __fmul2_rn(f2(cell0 < 0 || k0 == cell0 ? row_peak : 0.f), above(x0));
 #pragma unroll
             for (int j = 0; j < W2; ++j) {
-                const float2 v = __fadd2_rn(acc[j].h, f2(-B[j]));  // exact
+                const float2 v = minus(acc[j].h, B[j]);  // exact
                 const float2 s = __fadd2_rn(v, acc[j].l);
-                float top = fmaxf(fabsf(s.x), fabsf(s.y));
-                if (!finite(top)) {  // an infinite part stays what it is whatever the bias
-                    top = finite(s.x) ? fabsf(s.x) : 0.f;
-                    if (finite(s.y)) top = fabsf(s.y);
-                }
-                B[j] = bias((__float_as_int(fmaf(rx, kb.peak[j], top)) >> 23) - 125);
-                const float2 h = __fadd2_rn(s, f2(B[j]));
-                acc[j].l = __fadd2_rn(minus(acc[j].l, minus(s, v)),
-                                      minus(s, __fadd2_rn(h, f2(-B[j]))));
+                // (a part that is not finite stays what it is whatever its bias)
+                const float2 top = make_float2(finite(s.x) ? fabsf(s.x) : 0.f,
+                                               finite(s.y) ? fabsf(s.y) : 0.f);
+                B[j] = bias(__ffma2_rn(rx, f2(kb.peak[j]), top));
+                const float2 h = __fadd2_rn(s, B[j]);
+                acc[j].l = __fadd2_rn(minus(acc[j].l, minus(s, v)), minus(s, minus(h, B[j])));
                 acc[j].h = h;
             }
         }
@@ -535,7 +648,7 @@ __global__ void __launch_bounds__(kDsThreads, 3)
                 const bool need = (bm >> st) & 1u;
                 const int before = __shfl_sync(0xffffffffu, key, grp * W2 + max(st, 1) - 1);
                 const int fcell = st > 0 ? before : cell0;
-                const int xr = __shfl_sync(0xffffffffu, xe, grp * W2 + st);
+                const unsigned xr = __shfl_sync(0xffffffffu, xe, grp * W2 + st);
                 unsigned gm = __ballot_sync(0xffffffffu, need);
                 while (gm) {
                     const int g0 = (__ffs(gm) - 1) / W2;
@@ -690,7 +803,7 @@ static int degrid_ds(const lentils_plan *p, const double2 *grid, double2 *vis, c
                      const double *vscale)
 {
     const GridGeom &g = p->geom;
-    const size_t smem = sizeof(float4) * (size_t)g.E * g.stride + (size_t)g.E * g.T;
+    const size_t smem = sizeof(float4) * (size_t)g.E * g.stride + sizeof(uchar2) * (size_t)g.E * g.T;
     if (int st = ds_smem((const void *)degrid_ds_kernel<W2>, smem)) return st;
     LENTILS_CUDA_TRY(pdl_launch(degrid_ds_kernel<W2>, dim3(p->nitems), dim3(kDsThreads), smem, s,
                                 grid, (const uint2 *)p->coords, (const float2 *)p->coords_res, vis,
