@@ -82,8 +82,11 @@ __device__ __forceinline__ float2 recip2(float2 x)
 // x^(h0 + h1) for x > 0 and |h0| <= 1: x = 2^e m with m in [1/sqrt 2, sqrt 2),
 // log2 m = f P(f), f = m - 1, the exponent h (e + log2 m) split into an integer n and
 // a rest in [-1/2, 1/2] (h e - n by one fma, so it does not lose the low bits of a large
-// product), 2^rest by a polynomial, 2^n through the exponent field. P (degree 9, 2.1e-9) and
-// the exponential (degree 6, 3.0e-9) are Chebyshev fits of log2(1 + f) / f and 2^y.
+// product), 2^rest by a polynomial, 2^n through the exponent field. The coefficients are minimax fits
+// made one after the other from the constant term, each rounded to FP32 before the next: as they
+// stand here log2 m = f P(f) is within 1.5e-9 and 2^y within 3.0e-9 (relative), evaluated exactly.
+// A fixed error of the power moves all points near a radius the same way, so it is kept below the
+// rounding of single points.
 __device__ __forceinline__ float2 pow_pos(float2 x, float h0, float h1)
 {
     const int ix = __float_as_int(x.x), iy = __float_as_int(x.y);
@@ -94,14 +97,14 @@ __device__ __forceinline__ float2 pow_pos(float2 x, float h0, float h1)
     const float2 e = __fadd2_rn(make_float2(__int_as_float(0x4b400000 + ex),
                                             __int_as_float(0x4b400000 + ey)),
                                 splat(-12582912.f));
-    float2 p = splat(-0.11021894216537476f);
-    p = __ffma2_rn(p, f, splat(0.18633928894996643f));
-    p = __ffma2_rn(p, f, splat(-0.1910315454006195f));
-    p = __ffma2_rn(p, f, splat(0.20457172393798828f));
-    p = __ffma2_rn(p, f, splat(-0.23961789906024933f));
-    p = __ffma2_rn(p, f, splat(0.28856903314590454f));
-    p = __ffma2_rn(p, f, splat(-0.3606966733932495f));
-    p = __ffma2_rn(p, f, splat(0.4808982014656067f));
+    float2 p = splat(-0.10772465169429779f);
+    p = __ffma2_rn(p, f, splat(0.18571536242961884f));
+    p = __ffma2_rn(p, f, splat(-0.19199073314666748f));
+    p = __ffma2_rn(p, f, splat(0.2048441469669342f));
+    p = __ffma2_rn(p, f, splat(-0.23951542377471924f));
+    p = __ffma2_rn(p, f, splat(0.28853684663772583f));
+    p = __ffma2_rn(p, f, splat(-0.36070021986961365f));
+    p = __ffma2_rn(p, f, splat(0.4808996021747589f));
     p = __ffma2_rn(p, f, splat(-0.7213473320007324f));
     p = __ffma2_rn(p, f, splat(1.4426950216293335f));
     const float2 l = __fmul2_rn(p, f);  // log2 m
@@ -110,11 +113,11 @@ __device__ __forceinline__ float2 pow_pos(float2 x, float h0, float h1)
     const float2 tm = __fadd2_rn(__ffma2_rn(h, e, c), splat(12582912.f));  // rounds to integers
     const float2 nn = sub2(splat(12582912.f), tm);  // -n
     const float2 y = __fadd2_rn(__ffma2_rn(h, e, nn), c);
-    float2 r = splat(0.00015472411178052425f);
-    r = __ffma2_rn(r, y, splat(0.0013403140474110842f));
-    r = __ffma2_rn(r, y, splat(0.009618016891181469f));
-    r = __ffma2_rn(r, y, splat(0.055503204464912415f));
-    r = __ffma2_rn(r, y, splat(0.24022650718688965f));
+    float2 r = splat(0.00015326471475418657f);
+    r = __ffma2_rn(r, y, splat(0.0013390806270763278f));
+    r = __ffma2_rn(r, y, splat(0.009618505835533142f));
+    r = __ffma2_rn(r, y, splat(0.05550359934568405f));
+    r = __ffma2_rn(r, y, splat(0.24022647738456726f));
     r = __ffma2_rn(r, y, splat(0.6931471824645996f));
     r = __ffma2_rn(r, y, splat(1.f));
     const float2 sc = make_float2(__int_as_float((__float_as_int(tm.x) << 23) + 0x3f800000),
