@@ -259,17 +259,46 @@ __device__ __forceinline__ void shear_alpha(const DevLens &L, float sx, float sy
     }
 }
 
+// Multipoles at a point whose squared distance from the centre is not a normal FP32 number: the
+// same sums by a scaled offset and the library's functions. Not inlined: rare.
+static __device__ __noinline__ float2 multipole_scaled(const DevLens &L, float sx, float sy)
+{
+    if (L.order < 3) return make_float2(0.f, 0.f);
+    const float up = 0x1p+100f, top = fmaxf(fabsf(sx), fabsf(sy));
+    const float k = top < 1.f ? up : 1.f / up;
+    const float x = sx * k, y = sy * k, r = sqrtf(fmaf(x, x, y * y));
+    const float cn = x / r, sn = y / r;
+    const float h = 2.f * (L.h0 + L.h1);
+    const float rp = powf(r, h) * (k == up ? powf(1.f / up, h) : powf(up, h));
+    float cm = cn * cn - sn * sn, sm = 2.f * cn * sn, dr = 0.f, dt = 0.f;
+    for (int m = 3; m <= L.order; ++m) {
+        const float c = cm * cn - sm * sn;
+        sm = cm * sn + sm * cn;
+        cm = c;
+        dr = fmaf(L.rc[m], cm, fmaf(L.rs[m], sm, dr));
+        dt = fmaf(L.tc[m], cm, fmaf(L.ts[m], sm, dt));
+    }
+    return make_float2(rp * (cn * dr - sn * dt), rp * (sn * dr + cn * dt));
+}
+
 // Internal multipoles: with e = (sx + i sy) / r, cos m th and sin m th are the parts of e^m
 // (one complex product per order, no angle), and r^(1 - alpha) = (r^2)^h, h = (1 - alpha) / 2.
+// A squared radius outside the normal FP32 numbers (r below 1.1e-19 or above 1.8e19) would make the
+// reciprocal root 0 or infinite: those points are done again by multipole_scaled.
 template <int NP>
 __device__ __forceinline__ void multipole_alpha(const DevLens &L, const float2 (&sx)[NP],
                                                 const float2 (&sy)[NP], float2 (&ax)[NP],
                                                 float2 (&ay)[NP])
 {
     float2 rp[NP], cn[NP], sn[NP], nsn[NP], cm[NP], sm[NP], dr[NP], dt[NP];
+    auto normal = [](float a, float b) {  // both
+        return fminf(a, b) >= 0x1p-126f && fmaxf(a, b) <= 3.402823466e38f;
+    };
+    bool all = true;
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
         const float2 r2 = __ffma2_rn(sx[q], sx[q], __fmul2_rn(sy[q], sy[q]));
+        all = all && normal(r2.x, r2.y);
         rp[q] = lens_power(L, r2);
         float2 ri;
         asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ri.x) : "f"(r2.x));
@@ -300,6 +329,22 @@ __device__ __forceinline__ void multipole_alpha(const DevLens &L, const float2 (
     for (int q = 0; q < NP; ++q) {
         ax[q] = __fmul2_rn(rp[q], __ffma2_rn(cn[q], dr[q], __fmul2_rn(nsn[q], dt[q])));
         ay[q] = __fmul2_rn(rp[q], __ffma2_rn(sn[q], dr[q], __fmul2_rn(cn[q], dt[q])));
+    }
+    if (!all) {
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            const float2 r2 = __ffma2_rn(sx[q], sx[q], __fmul2_rn(sy[q], sy[q]));
+            if (!normal(r2.x, r2.x)) {
+                const float2 a = multipole_scaled(L, sx[q].x, sy[q].x);
+                ax[q].x = a.x;
+                ay[q].x = a.y;
+            }
+            if (!normal(r2.y, r2.y)) {
+                const float2 a = multipole_scaled(L, sx[q].y, sy[q].y);
+                ax[q].y = a.x;
+                ay[q].y = a.y;
+            }
+        }
     }
 }
 
