@@ -21,6 +21,7 @@
 #include <new>
 #include <vector>
 
+#include "clean_grid.cuh"
 #include "common.cuh"
 #include "fft2d.cuh"
 
@@ -38,10 +39,11 @@ struct lentils_nufft {
                // apodisation inside (pad32 / pad64 hold their scratch); else cuFFT
     lentils::Fft2d fft32, fft64;
     // own: the grids that the adjoint accumulates into, zero between calls (fft2d_inverse leaves
-    // them so); not_zero: a call failed in between
+    // them so), beside grid32 / grid64, which the forward operator leaves full; dirty: see
+    // accumulate_clean
     float2 *acc32;
     double2 *acc64;
-    bool not_zero32, not_zero64;
+    bool dirty32, dirty64;
     cufftHandle r2c32, c2r32, d2z64, z2d64;
     bool have32, have64;
 };
@@ -357,16 +359,27 @@ int nufft_forward_scaled64(lentils_nufft *op, const double *image, double *vis_p
 
 // Adjoint with the transforms of fft2d.cu.
 template <typename R, typename C, class Grid>
-static int own_adjoint(lentils_nufft *op, const Fft2d &fft, C *acc, bool &not_zero, const C *vis,
+static int own_adjoint(lentils_nufft *op, const Fft2d &fft, C *acc, bool &dirty, const C *vis,
                        C *mid, R *image, const R *apx, const R *apy, Grid launch, cudaStream_t s)
 {
-    if (not_zero)  // after a failed call
-        LENTILS_CUDA_TRY(cudaMemsetAsync(acc, 0, sizeof(C) * (size_t)op->nu * op->half_nv, s));
-    not_zero = true;
-    if (int st = launch(op->plan, vis, acc, s)) return st;
-    if (int st = fft2d_inverse<R, C>(fft, acc, mid, image, apx, apy, s)) return st;
-    not_zero = false;
-    return LENTILS_OK;
+    return accumulate_clean(
+        dirty,
+        [&]() -> int {
+            if (int st = launch(op->plan, vis, acc, s)) return st;
+            return fft2d_inverse<R, C>(fft, acc, mid, image, apx, apy, s);
+        },
+        [&]() -> int {
+            const size_t bytes = sizeof(C) * (size_t)op->nu * op->half_nv;
+            if (cudaMemsetAsync(acc, 0, bytes, s) == cudaSuccess) return LENTILS_OK;
+            // (behind a failed call its own message stays)
+            return dirty ? set_error(LENTILS_ERR_CUDA, "nufft_adjoint: clearing the grid")
+                         : LENTILS_ERR_CUDA;
+        },
+        [&] {
+            cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+            return cudaStreamIsCapturing(s, &status) == cudaSuccess &&
+                   status != cudaStreamCaptureStatusNone;
+        });
 }
 
 }  // namespace lentils
@@ -380,7 +393,7 @@ int lentils_nufft_adjoint(lentils_nufft *op, const float *vis_plan, float *image
         return set_error(LENTILS_ERR_INVALID, "nufft_adjoint: bad arguments (FP32 not created?)");
     cudaStream_t s = (cudaStream_t)stream;
     if (op->own)
-        return own_adjoint<float, float2>(op, op->fft32, op->acc32, op->not_zero32,
+        return own_adjoint<float, float2>(op, op->fft32, op->acc32, op->dirty32,
                                           (const float2 *)vis_plan, (float2 *)op->pad32, image,
                                           op->apx32, op->apy32, launch_grid, s);
     LENTILS_CUDA_TRY(cudaMemsetAsync(op->grid32, 0, sizeof(float2) * (size_t)op->nu * op->half_nv, s));
@@ -404,7 +417,7 @@ int lentils_nufft_adjoint64(lentils_nufft *op, const double *vis_plan, double *i
         return set_error(LENTILS_ERR_INVALID, "nufft_adjoint64: bad arguments (FP64 not created?)");
     cudaStream_t s = (cudaStream_t)stream;
     if (op->own)
-        return own_adjoint<double, double2>(op, op->fft64, op->acc64, op->not_zero64,
+        return own_adjoint<double, double2>(op, op->fft64, op->acc64, op->dirty64,
                                             (const double2 *)vis_plan, (double2 *)op->pad64,
                                             image, op->apx64, op->apy64, launch_grid64, s);
     LENTILS_CUDA_TRY(cudaMemsetAsync(op->grid64, 0, sizeof(double2) * (size_t)op->nu * op->half_nv, s));
