@@ -177,7 +177,7 @@ typedef struct {
     double gcx, gcy;     /* phase centre (radians)                                           */
     int wsup;            /* kernel half-width w, 1 <= w <= 8                                 */
     double kb_beta;      /* Kaiser-Bessel shape parameter                                    */
-    int tile;            /* tile edge in cells (16, 32 or 64), 0 = choose automatically      */
+    int tile;            /* tile edge in cells (8, 16, 32 or 64), 0 = choose automatically   */
     int chunk;           /* max visibilities per work item, 0 = choose automatically         */
 } lentils_grid_desc;
 

@@ -639,6 +639,43 @@ static int ensure_staging(lentils_plan *p)
     return LENTILS_OK;
 }
 
+// Tile. A work item pays for its extended tile -- staging or clearing, summing and flushing
+// (T + 2w)^2 cells -- whatever it holds, so 16-cell tiles win where the grid has many tiles or few
+// visibilities per tile, and the more the wider the kernel. On a small grid there are too few of
+// them to fill the SMs, and the ones around the centre are long: 8-cell tiles win there. Degrid +
+// grid in us, 8 against 16 cells, FP32 and FP64:
+//   w = 4     128^2, 2e4: 18 / 22, 27 / 33; 512^2, 5e5: 37 / 41, 108 / 131; 691^2, 3e5: 31 / 33,
+//             94 / 107; 691^2, 6.6e4: 23 / 21, 56 / 56; 1024^2, 2e6: 84 / 82, 336 / 360
+//   w = 6     256^2, 1.3e5: 24 / 27, 290 / 314; 512^2, 5e5: 53 / 57, 980 / 1064; 691^2, 5e5: 68 / 64;
+//             512^2, 2e4: 23 / 25, 140 / 132
+//   w = 8     256^2, 1.3e5: 27 / 35, 424 / 426; 340^2, 3e5: 43 / 51, 891 / 873; 512^2, 6.6e4: 31 / 31,
+//             398 / 276: a plan serves both types, and the FP64 kernels lose more
+static int default_tile(int w, long long cells, long long nvis)
+{
+    if (w <= 4)
+        return cells <= 550LL * 550 || (cells <= 700LL * 700 && 4 * nvis >= cells) ? 8 : 16;
+    return w <= 6 && cells <= 550LL * 550 && nvis >= cells ? 8 : 16;
+}
+
+// Work-item size: long items amortise their tile, but the longest must not outlast the rest. A few
+// hundred items for small problems, four per SM for large ones.
+//   8-cell tiles, w <= 4: 256^2, 2e4 visibilities: 8.4 us of FP32 degrid + grid with 64 per item, 9.3
+//   with 256. w > 4, whose items take longer per visibility: 128^2, 2e4, FP64: 88 us with 256 (w = 6),
+//   98 with 66; 340^2, 3e5: 600 with 375, 700 with 1000.
+//   16-cell tiles, mean over 720^2 to 1400^2 and w = 2 to 4, FP32 and FP64, against nvis / 608 or 256:
+//   1e5 visibilities: 1.00 and 1.06 with 384, 1.05 and 1.22 with 1024; 2e5: 0.98 and 0.98 with 384, 0.99
+//   and 1.11 with 1024; 4e5: 0.99 and 0.98 with 768. 1e7 on 2048^2: 264 us with 4096, 286 with 2048.
+//   w = 8: 340^2, 3e5, FP32 and FP64: 51 and 875 us with 493, 53 and 1012 with 600.
+static int default_chunk(int w, int T, long long nvis)
+{
+    const auto clamp = [](long long v, long long lo, long long hi) {
+        return (int)std::max(lo, std::min(hi, v));
+    };
+    if (T == 8 && w <= 4) return std::max(clamp(nvis / 300, 64, 1024), clamp(nvis / 1000, 0, 4096));
+    if (T == 8) return clamp(nvis / 800, 256, 4096);
+    return std::max(clamp(w <= 4 ? nvis / 500 : 0, 256, 1024), clamp(nvis / (4 * 152), 0, 4096));
+}
+
 }  // namespace lentils
 
 using namespace lentils;
@@ -672,31 +709,13 @@ int lentils_plan_create(lentils_plan **out, const lentils_grid_desc *gd, const d
     memset(p, 0, sizeof(*p));
     p->desc = *gd;
     cudaGetDevice(&p->device);
-    // Tile. A work item pays for its extended tile -- staging or clearing, summing and flushing
-    // (T + 2w)^2 cells -- whatever it holds, so 16-cell tiles win where the grid has many tiles
-    // (2048^2, 1e7 visibilities: degrid + grid 264 us against 300 with 8-cell tiles; 4e5
-    // visibilities: 62 against 99). On a small grid there are too few of them to fill the SMs,
-    // and the ones around the centre are long: 8-cell tiles win up to about 700^2 cells (256^2,
-    // 2e4: 8.4 us against 13.3; 500^2, 1.3e5: 14.9 against 17.1; 512^2, 5e5: 25.7 against 28.6;
-    // 512^2, 2e6: 54.7 against 60.8; 800^2: equal; 1024^2, 5e5: 39.8 against 36.2).
-    int T = gd->tile;
-    if (T == 0) T = (long long)gd->nu * gd->nv <= 700LL * 700 ? 8 : 16;
+    const int T = gd->tile ? gd->tile : default_tile(gd->wsup, (long long)gd->nu * gd->nv, nvis);
     const int logT = ilog2_exact(T);
     if (logT < 3 || logT > 6) {
         delete p;
         return set_error(LENTILS_ERR_INVALID, "plan_create: tile %d (use 8, 16, 32 or 64)", T);
     }
-    // Work-item size: long items amortise their tile, but the longest must not outlast the rest.
-    // A few hundred items for small problems, four per SM for large ones (256^2, 2e4: 8.4 us with
-    // 64 visibilities, 9.3 with 256; 800^2, 4e5: 30.5 us with 1024, 33.8 with 657, 36.6 with 2048;
-    // 1024^2, 1.6e6 in four channels: 97 us of degrid, grid and frames with 2631, 102 with 1600;
-    // 2048^2, 1e7: 264 us with 4096, 286 with 2048).
-    int chunk = gd->chunk;
-    if (chunk <= 0) {
-        const long long few = T == 8 ? std::max(64LL, std::min(1024LL, nvis / 300))
-                                     : std::min(1024LL, std::max(256LL, nvis / 64));
-        chunk = (int)std::max(few, std::min(4096LL, T == 8 ? nvis / 1000 : nvis / (4 * 152)));
-    }
+    const int chunk = gd->chunk > 0 ? gd->chunk : default_chunk(gd->wsup, T, nvis);
     p->desc.tile = T;
     p->desc.chunk = chunk;
     GridGeom &g = p->geom;
