@@ -821,7 +821,7 @@ def cpu_cg_baseline(inv, geom, budget_s=60.0):
 
 
 SWEEP_SEED = SEED + 3
-SWEEP_FORM = 0  # lentils_sweep_create flags: the sweep kernel's item functions
+SWEEP_FORM = 0  # lentils_sweep_create flags: one kernel per kind of work and KB table
 
 
 def run_sweep_bench(peak, nsamples=256, steps=10, warmup=3, form=SWEEP_FORM):
@@ -829,8 +829,8 @@ def run_sweep_bench(peak, nsamples=256, steps=10, warmup=3, form=SWEEP_FORM):
     sizes from {128, 256, 384, 512}^2 (0.02" pixels), visibility counts log-uniform in
     [1e5, 2e6] (uv density ~ 1/|uv| to 0.45 of Nyquist), per-sample KB width from the accuracy
     target 0.01 / sqrt(N_vis), tile and work-item size from the autotuner (JSON cache). One run
-    = deflection of every pixel grid + degrid + grid of every sample in one persistent launch,
-    replayed as a CUDA graph; timed with events on the sweep's stream. For comparison the same
+    = deflection of every pixel grid + degrid + grid of every sample in one CUDA graph (a kernel
+    per kind of work and KB table, on three branches); timed with events on the sweep's stream. For comparison the same
     work as separate per-sample launches (deflection, degrid, grid: three launches a sample)."""
     import numpy as np
     import torch
@@ -880,15 +880,15 @@ def run_sweep_bench(peak, nsamples=256, steps=10, warmup=3, form=SWEEP_FORM):
     tiles = [x.info["tile"] for x in samples]
     achieved = st["algorithmic_bytes"] / (ms * 1e-3) / 1e9
     return {"workload": f"{nsamples} PEMD+shear samples, images {{128..512}}^2, nvis log-uniform "
-                        "[1e5, 2e6]; deflection + degrid + grid per sample in one persistent "
-                        "launch (CUDA graph)",
+                        "[1e5, 2e6]; deflection + degrid + grid per sample in one CUDA "
+                        "graph",
             "seed": SWEEP_SEED, "total_vis": st["total_vis"], "total_pixels": st["total_pixels"],
             "ms_per_sweep": ms, "samples_per_s": nsamples / (ms * 1e-3),
             "mvis_per_s": st["total_vis"] / (ms * 1e-3) / 1e6,
             "note": "mvis_per_s = visibilities / (time of the whole sweep: degrid + grid of every "
                     "visibility and the deflections), the headline's convention",
             "per_sample_launches_ms": ms_sep, "speedup_vs_per_sample_launches": ms_sep / ms,
-            "work_items": st["nwork"], "persistent_ctas": st["blocks"],
+            "work_items": st["nwork"], "ctas": st["blocks"],
             "smem_bytes": st["smem_bytes"], "kb_width_counts": {"6": widths.count(6),
                                                                 "8": widths.count(8)},
             "tile_counts": {str(t): tiles.count(t) for t in sorted(set(tiles))},

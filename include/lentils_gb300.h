@@ -495,8 +495,8 @@ typedef struct {
 typedef struct {
     int nsamples;
     int nwork;        /* work items of all kinds                        */
-    int blocks;       /* CTAs of the persistent forms (resident slots on all SMs) */
-    long long smem_bytes; /* of the persistent forms, per CTA */
+    int blocks;       /* CTAs of one run: of all kernels of form 0, or of the persistent kernel */
+    long long smem_bytes; /* dynamic shared memory per CTA, of the kernel that has most */
     long long total_vis;
     long long total_pixels;
     double algorithmic_bytes; /* per run: 2 x (16 B per visibility + grid) + 8 B per pixel */

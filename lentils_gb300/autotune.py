@@ -13,10 +13,11 @@ degrid + grid pass with CUDA events (best of a few runs after a warm-up); the fa
 Results are stored per class in a JSON file (default lentils_gb300/tuning/<arch>.json, or the
 LENTILS_TUNING_CACHE path) and reused.
 
-Batched mode (mode="batched", for the persistent lens sweep) times every candidate inside the
-sweep kernel itself, on a small batch of synthetic samples of the class, because there the
-parallelism comes from the many samples: fewer, larger work items win where a single plan
-needs many small ones to fill the GPU. Its cache is <arch>_batched.json.
+Batched mode (mode="batched", for the lens sweep) times every candidate inside a sweep, on a small
+batch of synthetic samples of the class, because there the parallelism comes from the many
+samples: fewer, larger work items win where a single plan needs many small ones to fill the GPU.
+Its cache is <arch>_batched.json (the entries for sm_103 were timed in the sweep's persistent
+form).
 """
 from __future__ import annotations
 
@@ -133,7 +134,7 @@ class Autotuner:
                 "candidates": results}
 
     def tune_batched(self, nu, nv, du, dv, w2, nvis, nsamples=8, seed=0):
-        """Best (tile, chunk) for samples of this class inside the persistent sweep."""
+        """Best (tile, chunk) for samples of this class inside a sweep."""
         from .sweep import BatchedSweep, draw_samples
         rng = np.random.default_rng(seed)
         n = nu // 2

@@ -17,6 +17,7 @@
 // limit for three CTAs per SM, the faster item functions spill, and each item stages its table
 // in shared memory. 20 samples, 1.7e7 visibilities: 840 us persistent, 570 us split.
 #include <algorithm>
+#include <climits>
 #include <new>
 #include <vector>
 
@@ -481,7 +482,6 @@ int lentils_sweep_create(lentils_sweep **out, const lentils_sweep_sample *in, in
         }
         // the split form: this sample's items join the group of its table
         std::vector<int2> hchunks(p->nitems);
-        SweepGroup *grp = nullptr;
         if (p->nitems > 0 && (!p->chunk_begin || p->chunk_k != 4)) sw->split = false;
         if (sw->split) {
             size_t q = 0;
@@ -497,7 +497,7 @@ int lentils_sweep_create(lentils_sweep **out, const lentils_sweep_sample *in, in
                 }
             }
             if (sw->split) {
-                grp = &sw->groups[q];
+                SweepGroup *grp = &sw->groups[q];
                 grp->grid_smem = std::max(grp->grid_smem, w2 == 8
                                                               ? grid_pairs_smem_bytes<8, 4>(p->geom)
                                                               : grid_pairs_smem_bytes<6, 4>(p->geom));
@@ -533,36 +533,30 @@ int lentils_sweep_create(lentils_sweep **out, const lentils_sweep_sample *in, in
         delete sw;
         return st;
     }
-    std::stable_sort(items.begin(), items.end(),
-                     [](const std::pair<double, SweepWork> &a, const std::pair<double, SweepWork> &b) {
-                         return a.first > b.first;
-                     });
-    std::vector<SweepWork> hw(items.size());
-    for (size_t i = 0; i < items.size(); ++i) hw[i] = items[i].second;
     sw->nsamples = n;
-    sw->nwork = (int)hw.size();
-    sw->smem = std::max<size_t>(smem, 16);
+    sw->nwork = (int)items.size();
     cudaError_t e = cudaMalloc(&sw->samples, sizeof(SweepSampleDev) * std::max(1, n));
-    if (e == cudaSuccess) e = cudaMalloc(&sw->work, sizeof(SweepWork) * std::max<size_t>(1, hw.size()));
     if (e == cudaSuccess) e = cudaMalloc(&sw->lenses, sizeof(DevLens) * std::max<size_t>(1, hl.size()));
-    if (e == cudaSuccess) e = cudaMalloc(&sw->counter, sizeof(int));
     if (e == cudaSuccess && n > 0)
         e = cudaMemcpyAsync(sw->samples, hs.data(), sizeof(SweepSampleDev) * n, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess && !hw.empty())
-        e = cudaMemcpyAsync(sw->work, hw.data(), sizeof(SweepWork) * hw.size(), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess && !hl.empty())
         e = cudaMemcpyAsync(sw->lenses, hl.data(), sizeof(DevLens) * hl.size(), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = sweep_set_smem(sw->form, (int)sw->smem);
+    // sources of copies on s, as hs and hl: until the wait below
     std::vector<std::vector<SweepItem>> hgroups(sw->groups.size());
-    std::vector<int2> hchunk;  // sources of copies on s, as hs, hw and hl: until the wait below
+    std::vector<int2> hchunk;
+    std::vector<SweepWork> hw;
+    const auto longest = [](const auto &x, const auto &y) { return x.first > y.first; };
     if (sw->split) {
-        const auto longest = [](const auto &x, const auto &y) { return x.first > y.first; };
+        long long ctas = (long long)n * kZeroBlocks + (long long)chunks.size();
+        sw->smem = 0;
         for (size_t q = 0; q < sw->groups.size() && e == cudaSuccess; ++q) {
             SweepGroup &g = sw->groups[q];
             std::stable_sort(gitems[q].begin(), gitems[q].end(), longest);
             std::vector<SweepItem> &h = hgroups[q];
             for (const auto &x : gitems[q]) h.push_back(x.second);
             g.nitems = (int)h.size();
+            ctas += 2LL * g.nitems;
+            sw->smem = std::max(sw->smem, std::max(g.grid_smem, g.degrid_smem));
             e = cudaMalloc(&g.items, sizeof(SweepItem) * std::max<size_t>(1, h.size()));
             if (e == cudaSuccess && !h.empty())
                 e = cudaMemcpyAsync(g.items, h.data(), sizeof(SweepItem) * h.size(),
@@ -587,11 +581,24 @@ int lentils_sweep_create(lentils_sweep **out, const lentils_sweep_sample *in, in
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sw->join[k], cudaEventDisableTiming);
         }
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sw->fork, cudaEventDisableTiming);
+        sw->blocks = (int)std::min<long long>(INT_MAX, ctas);
+    } else {
+        std::stable_sort(items.begin(), items.end(), longest);
+        for (const auto &x : items) hw.push_back(x.second);
+        sw->smem = std::max<size_t>(smem, 16);
+        if (e == cudaSuccess) e = cudaMalloc(&sw->counter, sizeof(int));
+        if (e == cudaSuccess)
+            e = cudaMalloc(&sw->work, sizeof(SweepWork) * std::max<size_t>(1, hw.size()));
+        if (e == cudaSuccess && !hw.empty())
+            e = cudaMemcpyAsync(sw->work, hw.data(), sizeof(SweepWork) * hw.size(),
+                                cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = sweep_set_smem(sw->form, (int)sw->smem);
+        int per_sm = 0, nsm = 0, dev = 0;
+        if (e == cudaSuccess) e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess) e = sweep_occupancy(sw->form, &per_sm, sw->smem);
+        sw->blocks = std::max(1, std::min(sw->nwork, std::max(1, per_sm) * nsm));
     }
-    int per_sm = 0, nsm = 0, dev = 0;
-    if (e == cudaSuccess) e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = sweep_occupancy(sw->form, &per_sm, sw->smem);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
         st = cuda_status(e, "sweep_create");
@@ -599,7 +606,6 @@ int lentils_sweep_create(lentils_sweep **out, const lentils_sweep_sample *in, in
         delete sw;
         return st;
     }
-    sw->blocks = std::max(1, std::min(sw->nwork, std::max(1, per_sm) * nsm));
     *out = sw;
     return LENTILS_OK;
 }

@@ -4,10 +4,9 @@ whose operators run one lens model at a time).
 Each sample is a lens model (PEMD + external shear drawn from priors), an n x n image plane
 (pixel centres deflected to the source plane), and its own visibility set on the 2n x 2n
 r2c grid of that image; its KB width follows from its accuracy target (autotune.width_for)
-and its tile and work-item size from the autotuner (batched mode: timed inside the sweep
-kernel). One run degrids every sample's grid,
-grids every sample's visibilities and deflects every sample's pixel grid in one persistent
-kernel launch, replayed as a CUDA graph.
+and its tile and work-item size from the autotuner (batched mode: timed inside a sweep). One run
+degrids every sample's grid, grids every sample's visibilities and deflects every sample's pixel
+grid in one CUDA graph: a kernel per kind of work and KB table, on three branches.
 """
 from __future__ import annotations
 
