@@ -14,11 +14,15 @@
 // of each row of the visibility's own window, in gridding the sums so far and the largest of the
 // next visibilities of the same cell, so the rounding is relative to values that reach the same
 // results.
-// The weights are fits of degree 11 here (9 in the FP64 kernels, which differ from the profile
-// by 1.1e-10 of its peak at w = 4): within 1e-12 of the peak, so that the pairs' rounding does
-// not add to the fit's error but takes its place. F^T F of a 512^2 image with 2e6 visibilities
-// (w = 4): degridding 905 -> 128 us, gridding 1170 -> 211 us (the rest of the operator's 2410 ->
-// 580 us is its FFT, 340 -> 130); relative error against direct FP64 sums 8.6e-13 -> 2.7e-14.
+// The weights are fits of degree 11 here, 9 in the FP64 kernels. Largest difference from the
+// profile, in units of its peak, beta = 2.34 (2w), degree 11 and 9: w = 1: 3.9e-10 and 4.4e-8; 2:
+// 4.0e-11 and 5.0e-9; 3: 4.6e-12 and 5.4e-10; 4: 4.5e-13 and 1.1e-10 (the NUFFT's own beta at padding
+// 2 to 4: 2.5e-11 to 4.3e-10, 2.8e-11 to 1.0e-10, 4.0e-12 to 1.7e-11, 4.2e-13 to 3.1e-12). The
+// pairs' rounding, about 1e-14 of the result, is below that at every width, so the operators are
+// closer to the definition than in FP64 with the shorter fits, though a value has 48 bits for 53.
+// F^T F of a 512^2 image with 2e6 visibilities (w = 4): degridding 905 -> 137 us, gridding 1170 ->
+// 227 us (the rest of the operator's 2410 -> 586 us is its FFT, 340 -> 130); relative error against
+// direct FP64 sums 8.6e-13 -> 2.4e-14.
 //
 // Range. FP32 exponents do not cover FP64's, so a work item scales its tile (degrid) or its
 // visibilities (grid) by the power of two that brings the largest finite one to [1, 2) and the
