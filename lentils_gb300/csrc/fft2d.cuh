@@ -31,9 +31,9 @@ void fft2d_free(Fft2d *op);
 template <typename R, typename C>
 int fft2d_forward(const Fft2d &op, const R *img, C *mid, C *grid, const R *apx, const R *apy,
                   cudaStream_t s);
-// Half-plane spectrum -> image, and the spectrum is zero afterwards (crop of the unnormalised inverse, times the factors). The imaginary
-// parts of the self-conjugate columns (0 and nv / 2) of the column transforms do not count, as
-// in numpy's irfft2.
+// Half-plane spectrum -> image (crop of the unnormalised inverse, times the factors); the spectrum
+// is zero afterwards. The imaginary parts of the self-conjugate columns (0 and nv / 2) of the column
+// transforms do not count, as in numpy's irfft2.
 template <typename R, typename C>
 int fft2d_inverse(const Fft2d &op, C *grid, C *mid, R *img, const R *apx, const R *apy,
                   cudaStream_t s);

@@ -2561,7 +2561,7 @@ static int conv_persist(const bf16 *act, int C, int ks, int Bn, int H, int W, in
 // 4 TMA, 5 TMEM + MMA. Bound by that traffic, 11 KB per output row and 8 KB out again: 22.7 us
 // forward (with the output layer) and 20.5 us for the data gradient at batch 32 and 128^2; 35.4 and
 // 34.2 with three boxes per input row, one per horizontal tap, in bands of four rows.
-constexpr int kRowsPerSm = 4;  // fewest rows per SM: conv3_rows_ok
+constexpr int kRowsPerSm = 4;  // fewest rows per SM for this kernel: conv3_rows_ok
 constexpr int kRowSlots = 6;
 struct RowsSmem {
     static constexpr int kB = 9 * 2048, kRow = 130 * 64, kSlot = (kRow + 1023) / 1024 * 1024;
@@ -2763,8 +2763,12 @@ static int conv3_rows_launch(const bf16 *act, int Bn, int H, int flip, const bf1
 }
 
 // the row kernel for a convolution of Bn images of H x W: the shape it takes, and at least
-// kRowsPerSm rows of each image for every SM (a run of fewer rows loads more halo than it reuses);
-// with fewer (batch 1) the persistent GEMM's row tiles spread wider
+// kRowsPerSm rows for every SM; with fewer (batch 1) the persistent GEMM's row tiles spread wider.
+// The launch deals the rows out to three CTAs per SM, so a run has one or two rows at that limit (2.4
+// input rows per output row) and nine at batch 32 (1.2). One CTA per kRowsPerSm rows instead, with
+// runs twice as long at small batches, measured within 0.7 % of that (training step at batch 5
+// to 32: 233.4 and 233.9 us, 247.4 and 249.0, 296.1 and 292.8 at 12, 462.1 and 462.3): the CTAs
+// more hide what the halo costs
 static bool conv3_rows_ok(int C, int N, int ks, int W, int Bn, int H)
 {
     return C == 32 && N == 32 && ks == 3 && W == 128 &&
