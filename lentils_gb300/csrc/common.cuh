@@ -151,6 +151,11 @@ __device__ __forceinline__ void pdl_entry()
 // A kernel that starts while they drain gets more of its first (longest) CTAs onto the SMs that
 // drain first; dealt out to idle SMs its work is balanced.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// the start of the next kernel, by a kernel that began with pdl_wait
+__device__ __forceinline__ void pdl_trigger()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 template <class... KArgs, class... Args>
 inline cudaError_t pdl_launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
@@ -172,6 +177,9 @@ inline cudaError_t pdl_launch_cluster(void (*kern)(KArgs...), dim3 grid, dim3 bl
     cfg.numAttrs = cluster.x * cluster.y * cluster.z > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
+
+// SMs; a grid of more CTAs than that has several per SM
+constexpr unsigned kSMs = 152;
 
 template <class... KArgs, class... Args>
 inline cudaError_t pdl_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,

@@ -244,6 +244,37 @@ __device__ __forceinline__ int fft_at(int t, int i)
     return t + (i / R) * S::T + (i % R) * (N / R);
 }
 
+// Programmatic dependent launch. FP32 transforms are latency chains, and let the next kernel start as
+// soon as they have all begun. FP64 ones are bound by the FP64 pipe of the SMs that they run on,
+// and a kernel that starts while another still holds most SMs has its CTAs packed onto the SMs that
+// are free: the row pass of a 512^2 plane (128 CTAs of a warp) took 75 us for 24. So they let the next
+// kernel start when their results are ready (fft_end), and a grid of more CTAs than SMs starts on an
+// idle GPU (fft_launch). Early start everywhere, late start everywhere, this rule, no early start at
+// all, us per call, FP64: F of a 256^2 image with 6e4 visibilities, w = 3: 109, 53, 53, 61; F^T F of
+// 512^2 with 2e6, w = 4: 580, 563, 483, 486; of 128^2 with 2e4: 95, 84, 84, 98; the dirty-beam
+// convolution of 512^2: 250, 208, 127, 130; of 64^2: 56, 56, 56, 64.
+template <typename C>
+__device__ __forceinline__ void fft_begin()
+{
+    if constexpr (sizeof(C) == 8) pdl_entry();
+    else pdl_wait();
+}
+template <typename C>
+__device__ __forceinline__ void fft_end()  // before the stores
+{
+    if constexpr (sizeof(C) == 16) pdl_trigger();
+}
+template <typename C, class K, class... Args>
+static cudaError_t fft_launch(K kern, dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                              Args &&...args)
+{
+    if (sizeof(C) == 16 && grid.x > kSMs) {
+        kern<<<grid, block, smem, s>>>(std::forward<Args>(args)...);
+        return cudaGetLastError();
+    }
+    return pdl_launch(kern, grid, block, smem, s, std::forward<Args>(args)...);
+}
+
 template <int N>
 constexpr int kRowPairs = FftShape<N>::T >= 32 ? 1 : 32 / FftShape<N>::T;  // per CTA
 template <int N>
@@ -269,7 +300,7 @@ __global__ void __launch_bounds__(kRowPairs<N> *FftShape<N>::T)
         const int j = t + q * S::T - pady;
         f[q] = j >= 0 && j < ny ? (apy ? apy[j] : (R)1) : (R)0;
     }
-    pdl_entry();
+    fft_begin<C>();
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
         const int j = t + q * S::T - pady;
@@ -292,6 +323,7 @@ __global__ void __launch_bounds__(kRowPairs<N> *FftShape<N>::T)
 #pragma unroll
     for (int i = 0; i < 16; ++i) sm(fft_at<N>(t, i)) = v[i];
     __syncthreads();
+    fft_end<C>();
     // Z = A + iB with A, B Hermitian: A_k = (Z_k + conj Z_-k) / 2, B_k = (Z_k - conj Z_-k) / 2i
     constexpr int half = N / 2 + 1, pitch = fft2d_pitch(N);
 #pragma unroll
@@ -322,7 +354,7 @@ __global__ void __launch_bounds__(kRowPairs<N> *FftShape<N>::T)
     auto sm = [&](int pos) -> C & { return smem[w * S::PAD + pos + (pos >> 4)]; };
     constexpr int pitch = fft2d_pitch(N);
     const Twiddles<N, C> tws(tw, t);
-    pdl_entry();
+    fft_begin<C>();
     // Z_k = A_k + i B_k, Z_-k = conj A_k + i conj B_k; all loads before the first store
     C v[16];
     const C *ma = mid + (long long)a * pitch, *mb = mid + (long long)b * pitch;
@@ -354,6 +386,7 @@ __global__ void __launch_bounds__(kRowPairs<N> *FftShape<N>::T)
     for (int q = 0; q < 16; ++q) v[q] = sm(t + q * S::T);
     __syncthreads();
     fft_regs<N, true>(v, t, tws, sm);
+    fft_end<C>();
     const R fa = a < nx ? (apx ? apx[a] : (R)1) : (R)0, fb = b < nx ? (apx ? apx[b] : (R)1) : (R)0;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -382,7 +415,7 @@ __global__ void __launch_bounds__(kCols<N> *FftShape<N>::T)
     const bool on = col < half;
     auto sm = [&](int pos) -> C & { return smem[(pos + (pos >> 4)) * NC + c]; };
     const Twiddles<N, C> tws(tw, t);
-    pdl_entry();
+    fft_begin<C>();
     C v[16];
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
@@ -414,6 +447,7 @@ __global__ void __launch_bounds__(kCols<N> *FftShape<N>::T)
         __syncthreads();
         fft_regs<N, true>(v, t, tws, sm);
     }
+    fft_end<C>();
     if (!on) return;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -475,11 +509,11 @@ static int rows(const Fft2d &op, bool inverse, const void *in, void *out, const 
     const dim3 block(kRowPairs<N> * FftShape<N>::T);
     const C *tw = (const C *)op.tw_v;
     if (inverse)
-        LENTILS_CUDA_TRY(pdl_launch(fft_rows_inverse<R, C, N>, grid, block, 0, s, (const C *)in,
-                                    (R *)out, apx, apy, tw, op.nx, op.ny, op.pady));
+        LENTILS_CUDA_TRY(fft_launch<C>(fft_rows_inverse<R, C, N>, grid, block, 0, s, (const C *)in,
+                                       (R *)out, apx, apy, tw, op.nx, op.ny, op.pady));
     else
-        LENTILS_CUDA_TRY(pdl_launch(fft_rows_forward<R, C, N>, grid, block, 0, s, (const R *)in,
-                                    (C *)out, apx, apy, tw, op.nx, op.ny, op.pady));
+        LENTILS_CUDA_TRY(fft_launch<C>(fft_rows_forward<R, C, N>, grid, block, 0, s, (const R *)in,
+                                       (C *)out, apx, apy, tw, op.nx, op.ny, op.pady));
     LENTILS_CHECK_LAUNCH("fft_rows");
     return LENTILS_OK;
 }
@@ -493,9 +527,9 @@ static int columns(const Fft2d &op, C *in, C *out, const C *spec, cudaStream_t s
         LENTILS_CUDA_TRY(cudaFuncSetAttribute(fft_columns<C, N, MODE>,
                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)smem));
-    LENTILS_CUDA_TRY(pdl_launch(fft_columns<C, N, MODE>, dim3((op.half + NC - 1) / NC),
-                                dim3(NC * FftShape<N>::T), smem, s, in, out, spec,
-                                (const C *)op.tw_u, op.nx, op.padx, op.half, op.pitch));
+    LENTILS_CUDA_TRY(fft_launch<C>(fft_columns<C, N, MODE>, dim3((op.half + NC - 1) / NC),
+                                   dim3(NC * FftShape<N>::T), smem, s, in, out, spec,
+                                   (const C *)op.tw_u, op.nx, op.padx, op.half, op.pitch));
     LENTILS_CHECK_LAUNCH("fft_columns");
     return LENTILS_OK;
 }

@@ -21,7 +21,7 @@
 // pairs' rounding, about 1e-14 of the result, is below that at every width, so the operators are
 // closer to the definition than in FP64 with the shorter fits, though a value has 48 bits for 53.
 // F^T F of a 512^2 image with 2e6 visibilities (w = 4): degridding 905 -> 137 us, gridding 1170 ->
-// 227 us (the rest of the operator's 2410 -> 586 us is its FFT, 340 -> 130); relative error against
+// 227 us (the rest of the operator's 2410 -> 495 us is its FFT, 340 -> 130); relative error against
 // direct FP64 sums 8.6e-13 -> 2.4e-14.
 //
 // Range. FP32 exponents do not cover FP64's, so a work item scales its tile (degrid) or its
@@ -210,6 +210,7 @@ __device__ __forceinline__ int block_max_exponent(int e, int *red)
     return m;
 }
 
+// (Both kernels let the next one start when they end, pdl_wait: see fft2d.cu.)
 constexpr int kDsThreads = 128;
 
 // Cell (ea, eb) of the extended tile at (a0, b0), through the Hermitian fold.
@@ -302,7 +303,7 @@ __global__ void __launch_bounds__(kDsThreads, W2 == 6 ? 3 : 4)  // 4 would spill
     uchar2 *rowmax = reinterpret_cast<uchar2 *>(sm + g.E * g.stride);
     __shared__ int red[kDsThreads / 32];
     constexpr int w = W2 / 2;
-    pdl_entry();
+    pdl_wait();
     const WorkItem it = items[blockIdx.x];
     const int a0 = it.tu * g.T - g.Hu - w, b0 = it.tv * g.T - g.Hv - w;
     const int E = g.E, S = g.stride;
@@ -450,7 +451,7 @@ __global__ void __launch_bounds__(kDsThreads, 3)
     constexpr int G = 32 / W2, NG = NW * G;
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ int red[NW];
-    pdl_entry();
+    pdl_wait();
     const WorkItem it = items[blockIdx.x];
     const int E = g.E, S = g.stride;
     float4 *tiles = reinterpret_cast<float4 *>(smraw);
