@@ -647,14 +647,15 @@ static int ensure_staging(lentils_plan *p)
 //   w = 4     128^2, 2e4: 18 / 22, 27 / 33; 512^2, 5e5: 37 / 41, 108 / 131; 691^2, 3e5: 31 / 33,
 //             94 / 107; 691^2, 6.6e4: 23 / 21, 56 / 56; 1024^2, 2e6: 84 / 82, 336 / 360
 //   w = 6     256^2, 1.3e5: 24 / 27, 290 / 314; 512^2, 5e5: 53 / 57, 980 / 1064; 691^2, 5e5: 68 / 64;
-//             512^2, 2e4: 23 / 25, 140 / 132
+//             512^2, 2e4: 23 / 25, 140 / 132; 256^2, 2e6: 130 / 134, 3757 / 3849; 65^2, 6e5, FP64:
+//             1296 / 1223
 //   w = 8     256^2, 1.3e5: 27 / 35, 424 / 426; 340^2, 3e5: 43 / 51, 891 / 873; 512^2, 6.6e4: 31 / 31,
 //             398 / 276: a plan serves both types, and the FP64 kernels lose more
 static int default_tile(int w, long long cells, long long nvis)
 {
     if (w <= 4)
         return cells <= 550LL * 550 || (cells <= 700LL * 700 && 4 * nvis >= cells) ? 8 : 16;
-    return w <= 6 && cells <= 550LL * 550 && nvis >= cells ? 8 : 16;
+    return w <= 6 && cells <= 550LL * 550 && nvis >= cells && nvis <= 32 * cells ? 8 : 16;
 }
 
 // Work-item size: long items amortise their tile, but the longest must not outlast the rest. A few

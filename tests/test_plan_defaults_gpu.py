@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
     (3, 128, 20000, 8, 66), (4, 256, 500000, 8, 1024), (4, 512, 10000, 8, 64),
     (4, 690, 300000, 8, 1000), (4, 690, 20000, 16, 256), (2, 720, 40000, 16, 256),
     (4, 1024, 100000, 16, 256), (3, 1024, 200000, 16, 400), (4, 1024, 2000000, 16, 3289),
-    (5, 256, 131072, 8, 256), (6, 512, 500000, 8, 625), (6, 256, 30000, 16, 256),
+    (5, 256, 131072, 8, 256), (6, 512, 500000, 8, 625), (6, 256, 30000, 16, 256), (6, 65, 600000, 16, 986),
     (6, 690, 500000, 16, 822), (8, 128, 20000, 16, 256), (8, 340, 300000, 16, 493)])
 def test_defaults(native, w, n, nvis, tile, chunk):
     from lentils_gb300.gridding import GriddingPlan
