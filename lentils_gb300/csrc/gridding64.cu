@@ -592,6 +592,7 @@ __global__ void __launch_bounds__(kDsThreads, 3)
         // visibilities beyond the range: in FP64, straight to the grid, the taps over the lanes
         for (unsigned fm = __ballot_sync(0xffffffffu, fx.x != 0.0 || fx.y != 0.0); fm;
              fm &= fm - 1) {
+            __syncwarp();  // the rows are written
             const int src = __ffs(fm) - 1;
             const double xr = __shfl_sync(0xffffffffu, fx.x, src);
             const double xi = __shfl_sync(0xffffffffu, fx.y, src);
